@@ -60,7 +60,8 @@ void count_launch(long k = 1);
 
 // Ensure a device exists and the runtime is usable; throws DG_ERR_NODEVICE otherwise.
 void require_device();
-// Per-thread library stream (non-blocking with respect to the legacy stream).
+// Per-thread library stream (non-blocking with respect to the legacy stream); a thread that ends
+// hands it to the next one.
 cudaStream_t stream();
 int sm_count();
 
@@ -85,8 +86,8 @@ struct PoolHold {
 void *pool_alloc(size_t bytes, cudaStream_t st);
 void pool_free(void *p, cudaStream_t st);
 
-// Mapped pinned host memory is kept in a small per-thread cache of blocks for the same
-// reason (cudaHostAlloc / cudaFreeHost cost far more than one solver step).
+// Mapped pinned host memory is kept in a bounded list of blocks, shared by all threads, for the
+// same reason (cudaHostAlloc / cudaFreeHost cost far more than one solver step).
 void *mapped_acquire(size_t bytes, size_t *got);
 void mapped_return(void *h, size_t bytes);
 

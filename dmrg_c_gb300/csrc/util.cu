@@ -33,21 +33,72 @@ void require_device() {
   }
 }
 
+// ---- streams ----------------------------------------------------------------------------
+// A thread's stream goes back to its device's list when the thread ends, and the next thread
+// takes it from there.  The worker threads of the batched and served forms live for one call or
+// one engine; with a stream created for each of them and never given back, every stream a
+// process had ever used stayed in the driver's list that a stream-ordered allocation walks:
+// after ~100 batched calls of 9 threads each a resident expectation value took 10.5 ms instead
+// of 0.25 ms and a batched solve of 24 chains 76 ms instead of 27.
+namespace {
+constexpr int kMaxPoolDevices = 64;
+constexpr size_t kKeptStreams = 64;   // idle streams kept per device; more are destroyed
+struct IdleStreams {
+  std::mutex mu;
+  std::vector<cudaStream_t> idle[kMaxPoolDevices];
+};
+// never destroyed: threads may end after static destruction has begun
+IdleStreams &idle_streams() {
+  static IdleStreams *s = new IdleStreams();
+  return *s;
+}
+struct ThreadStream {
+  cudaStream_t s = nullptr;
+  int dev = -1;
+  void give_back() {
+    if (!s) return;
+    // work still queued on it stays in order before the next owner's
+    bool kept = false;
+    if (dev >= 0 && dev < kMaxPoolDevices) {
+      IdleStreams &is = idle_streams();
+      std::lock_guard<std::mutex> lk(is.mu);
+      if (is.idle[dev].size() < kKeptStreams) {
+        is.idle[dev].push_back(s);
+        kept = true;
+      }
+    }
+    if (!kept) cudaStreamDestroy(s);
+    s = nullptr;
+  }
+  void take(int device) {
+    if (device >= 0 && device < kMaxPoolDevices) {
+      IdleStreams &is = idle_streams();
+      std::lock_guard<std::mutex> lk(is.mu);
+      if (!is.idle[device].empty()) {
+        s = is.idle[device].back();
+        is.idle[device].pop_back();
+      }
+    }
+    if (!s) DG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    dev = device;
+  }
+  ~ThreadStream() { give_back(); }
+};
+}  // namespace
+
 cudaStream_t stream() {
-  thread_local cudaStream_t s = nullptr;
-  thread_local int dev = -1;
+  thread_local ThreadStream t;
   int cur = 0;
   DG_CUDA(cudaGetDevice(&cur));
-  if (!s || dev != cur) {
-    DG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    dev = cur;
+  if (!t.s || t.dev != cur) {
+    t.give_back();
+    t.take(cur);
   }
-  return s;
+  return t.s;
 }
 
 // ---- device memory pool ---------------------------------------------------------------
 namespace {
-constexpr int kMaxPoolDevices = 64;
 std::mutex g_pool_mutex;
 cudaMemPool_t g_pools[kMaxPoolDevices] = {nullptr};
 
@@ -117,46 +168,62 @@ void pool_free(void *p, cudaStream_t st) {
 }
 
 // ---- mapped host blocks ------------------------------------------------------------------
+// One list for the process: a block returned by one thread serves the next solve of any thread
+// (a worker thread of the batched form lives for one call; with a list per thread it allocated
+// its blocks anew and freed them at its end, and freeing pinned memory waits for the device).
 namespace {
 struct MappedBlock {
   void *h;
   size_t bytes;
 };
-struct MappedCache {
-  std::vector<MappedBlock> free_blocks;
-  ~MappedCache() {
-    for (auto &b : free_blocks) cudaFreeHost(b.h);
-  }
+constexpr size_t kKeptBlocks = 256, kKeptBlockBytes = size_t(64) << 20;   // more are freed
+struct MappedList {
+  std::mutex mu;
+  std::vector<MappedBlock> idle;
+  size_t bytes = 0;
 };
-thread_local MappedCache g_mapped_cache;
+MappedList &mapped_list() {   // never destroyed, as idle_streams()
+  static MappedList *l = new MappedList();
+  return *l;
+}
 }  // namespace
 
 void *mapped_acquire(size_t bytes, size_t *got) {
   size_t want = 4096;
   while (want < bytes) want <<= 1;
-  auto &fb = g_mapped_cache.free_blocks;
-  for (size_t i = 0; i < fb.size(); ++i) {
-    if (fb[i].bytes >= want) {
-      MappedBlock b = fb[i];
-      fb.erase(fb.begin() + (long)i);
+  {
+    MappedList &l = mapped_list();
+    std::lock_guard<std::mutex> lk(l.mu);
+    size_t best = l.idle.size();   // the smallest block that fits
+    for (size_t i = 0; i < l.idle.size(); ++i)
+      if (l.idle[i].bytes >= want && (best == l.idle.size() || l.idle[i].bytes < l.idle[best].bytes)) best = i;
+    if (best < l.idle.size()) {
+      const MappedBlock b = l.idle[best];
+      l.idle[best] = l.idle.back();
+      l.idle.pop_back();
+      l.bytes -= b.bytes;
       *got = b.bytes;
       return b.h;
     }
   }
   void *h = nullptr;
-  DG_CUDA(cudaHostAlloc(&h, want, cudaHostAllocMapped));
+  DG_CUDA(cudaHostAlloc(&h, want, cudaHostAllocMapped | cudaHostAllocPortable));
   *got = want;
   return h;
 }
 
 void mapped_return(void *h, size_t bytes) {
   if (!h) return;
-  auto &fb = g_mapped_cache.free_blocks;
-  if (fb.size() >= 16) {
-    cudaFreeHost(h);
-    return;
+  {
+    MappedList &l = mapped_list();
+    std::lock_guard<std::mutex> lk(l.mu);
+    if (l.idle.size() < kKeptBlocks && l.bytes + bytes <= kKeptBlockBytes) {
+      l.idle.push_back(MappedBlock{h, bytes});
+      l.bytes += bytes;
+      return;
+    }
   }
-  fb.push_back(MappedBlock{h, bytes});
+  cudaFreeHost(h);
 }
 
 int sm_count() {
