@@ -8,10 +8,12 @@
 // by row (the row of M1 scattered, each column of W summed in its storage order, |value| > 1e-15
 // kept, CRS).  On the device both products are one thread per output entry over dense copies of the
 // scattered operand -- M3 by columns, M1 by columns -- with the sums in the reference's order and
-// rounded as written, so every kept value is bitwise the reference's; an ordered compaction (a
+// rounded as written, so every kept value is bitwise the reference's (entries whose operands' supports
+// lie apart are zero and cost no sum); an ordered compaction (a
 // block per column of W / row of Out, prefix sums of the keep flags) writes CCS / CRS in the
 // reference's element order.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -23,47 +25,122 @@ namespace {
 
 constexpr double kZero = 1e-15;   // |value| above this is kept (pow(10,-15) in the reference)
 
-// D[c * ld + row] = value, column by column in storage order (the last of repeated rows wins, as in
-// the reference's scatter).  ptr has ncol+1 offsets.
-__global__ void k_scatter_cols(int ncol, const int64_t *__restrict__ ptr, const int *__restrict__ idx, const double *__restrict__ val,
-                               int64_t ld, double *__restrict__ D) {
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncol; c += gridDim.x * blockDim.x)
-    for (int64_t e = ptr[c]; e < ptr[c + 1]; ++e) D[(int64_t)c * ld + idx[e]] = val[e];
-}
+// Support of a line (a column of M3, a row of M1 or M2): the smallest and largest index stored,
+// (INT_MAX, -1) for an empty one.
+struct Span {
+  int lo, hi;
+};
+__device__ __forceinline__ bool apart(Span a, Span b) { return a.lo > b.hi || a.hi < b.lo; }
 
-// D[col * ld + r] = value for the entries of row r, row by row in storage order (a transposed dense
-// copy: threads of consecutive r then read consecutive addresses).
-__global__ void k_scatter_rows_t(int nrow, const int64_t *__restrict__ ptr, const int *__restrict__ idx, const double *__restrict__ val,
-                                 int64_t ld, double *__restrict__ D) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nrow; r += gridDim.x * blockDim.x)
-    for (int64_t e = ptr[r]; e < ptr[r + 1]; ++e) D[(int64_t)idx[e] * ld + r] = val[e];
-}
-
-// W[c * rows + i] = sum over row i of M2 (storage order) of D3[c * ld3 + col] * val.
-__global__ void __launch_bounds__(kThreads) k_rows_times_dense(int rows, int ncols, const int64_t *__restrict__ rp, const int *__restrict__ ci,
-                                                              const double *__restrict__ cv, const double *__restrict__ D, int64_t ld,
-                                                              double *__restrict__ W) {
-  const int64_t total = (int64_t)rows * ncols;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(e / rows), i = (int)(e - (int64_t)c * rows);
-    const double *__restrict__ d = D + (int64_t)c * ld;
-    double acc = 0.0;
-    for (int64_t k = rp[i]; k < rp[i + 1]; ++k) acc = __dadd_rn(acc, __dmul_rn(d[ci[k]], cv[k]));
-    W[e] = acc;
+// The spans of n lines and, with D, their dense copy: entry e of line l goes to
+// D[l * lstride + idx[e] * estride], in storage order (the last of repeated indices wins, as in the
+// reference's scatter; within 32 entries the highest lane of an index writes).  *odd is set when a
+// value is infinite or NaN.  A warp per line: with one thread a line, each walking its entries
+// through two dependent L2 round trips, the scatters of T (512 lines of ~36) took 109 and 101 us;
+// now about 5.
+__global__ void __launch_bounds__(kThreads) k_lines(int n, const int64_t *__restrict__ ptr, const int *__restrict__ idx,
+                                                   const double *__restrict__ val, Span *__restrict__ span, double *__restrict__ D,
+                                                   int64_t lstride, int64_t estride, int *__restrict__ odd) {
+  const int lane = threadIdx.x & 31;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  for (int l = warp; l < n; l += nw) {
+    const int64_t b = ptr[l], e = ptr[l + 1];
+    unsigned lo = INT_MAX;
+    int hi = -1;
+    bool bad = false;
+    for (int64_t k0 = b; k0 < e; k0 += 32) {
+      const int64_t k = k0 + lane;
+      const int i = k < e ? idx[k] : -1;
+      const double v = k < e ? val[k] : 0.0;
+      if (k < e) {
+        lo = min(lo, (unsigned)i);
+        hi = max(hi, i);
+        bad = bad || !isfinite(v);
+      }
+      if (D) {
+        const unsigned same = __match_any_sync(0xffffffffu, i);
+        if (k < e && 31 - __clz(same) == lane) D[(int64_t)l * lstride + (int64_t)i * estride] = v;
+        __syncwarp();   // the next 32 entries' stores come after these
+      }
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane == 0) span[l] = Span{(int)lo, hi};
+    if (__any_sync(0xffffffffu, bad) && lane == 0) *odd = 1;
   }
 }
 
-// O[c * rows + r] = sum over the stored entries of column c of W (storage order) of
-// D1[row * rows + r] * value.
+// W[c * rows + i] = sum over row i of M2 (storage order) of D3[c * ld3 + col] * val.  A block per
+// column, a thread per row.  Where the row's columns lie apart from the support of M3's column every
+// product is a zero, which changes no sum: the entry is 0 without walking the row.  The operands of a
+// renormalisation conserve the block labels, so that is nine entries of ten, and the FP64 work (two
+// instructions a term, rounded apart) is what bounds the rest: Hubbard m=512 (2048 x 512 entries,
+// 74 k stored in M2) 213 us with every row walked; the whole call from host arrays 0.95 -> 0.55 ms.  A product of zero and an infinity is not zero:
+// when M2 holds a non-finite value (odd) every row is walked.
+__global__ void __launch_bounds__(kThreads) k_rows_times_dense(int rows, int ncols, const int64_t *__restrict__ rp, const int *__restrict__ ci,
+                                                              const double *__restrict__ cv, const Span *__restrict__ rspan,
+                                                              const Span *__restrict__ cspan, const int *__restrict__ odd,
+                                                              const double *__restrict__ D, int64_t ld, double *__restrict__ W,
+                                                              int *__restrict__ w_odd) {
+  const bool walk_all = *odd != 0;
+  for (int c = blockIdx.y; c < ncols; c += gridDim.y) {
+    const double *__restrict__ d = D + (int64_t)c * ld;
+    const Span sc = cspan[c];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) {
+      double acc = 0.0;
+      if (walk_all || !apart(rspan[i], sc)) {
+        int64_t k = rp[i];
+        const int64_t e = rp[i + 1];
+        for (; k + 8 <= e; k += 8) {   // eight gathers in flight, summed in storage order
+          int cc[8];
+          double a[8], v[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            cc[u] = ci[k + u];
+            v[u] = cv[k + u];
+          }
+#pragma unroll
+          for (int u = 0; u < 8; ++u) a[u] = d[cc[u]];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) acc = __dadd_rn(acc, __dmul_rn(a[u], v[u]));
+        }
+        for (; k < e; ++k) acc = __dadd_rn(acc, __dmul_rn(d[ci[k]], cv[k]));
+        if (!isfinite(acc)) *w_odd = 1;
+      }
+      W[(int64_t)c * rows + i] = acc;
+    }
+  }
+}
+
+// O[c * rows + r] = sum over the stored entries of column c of W (storage order, rows ascending) of
+// D1[row * rows + r] * value; 0 where the column's rows lie apart from row r of M1's columns (as
+// k_rows_times_dense; w_odd: W holds a non-finite value).
 __global__ void __launch_bounds__(kThreads) k_dense_times_cols(int rows, int ncols, const int64_t *__restrict__ cp,
                                                               const int *__restrict__ ri, const double *__restrict__ rv,
+                                                              const Span *__restrict__ rspan, const int *__restrict__ w_odd,
                                                               const double *__restrict__ D1, double *__restrict__ O) {
-  const int64_t total = (int64_t)rows * ncols;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(e / rows), r = (int)(e - (int64_t)c * rows);
-    double acc = 0.0;
-    for (int64_t k = cp[c]; k < cp[c + 1]; ++k) acc = __dadd_rn(acc, __dmul_rn(D1[(int64_t)ri[k] * rows + r], rv[k]));
-    O[e] = acc;
+  const bool walk_all = *w_odd != 0;
+  for (int c = blockIdx.y; c < ncols; c += gridDim.y) {
+    const int64_t b = cp[c], e = cp[c + 1];
+    const Span sc = e > b ? Span{ri[b], ri[e - 1]} : Span{INT_MAX, -1};
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) {
+      double acc = 0.0;
+      if (walk_all || !apart(rspan[r], sc)) {
+        int64_t k = b;
+        for (; k + 8 <= e; k += 8) {
+          double a[8], v[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            a[u] = D1[(int64_t)ri[k + u] * rows + r];
+            v[u] = rv[k + u];
+          }
+#pragma unroll
+          for (int u = 0; u < 8; ++u) acc = __dadd_rn(acc, __dmul_rn(a[u], v[u]));
+        }
+        for (; k < e; ++k) acc = __dadd_rn(acc, __dmul_rn(D1[(int64_t)ri[k] * rows + r], rv[k]));
+      }
+      O[(int64_t)c * rows + r] = acc;
+    }
   }
 }
 
@@ -175,13 +252,22 @@ void crs_crs_ccs(CRS1 *M1, CRS1 *M2, CCS1 *M3, CRS1 *Out, CCS1 *Work, double *Wo
     upload(d_v3, M3->Val + M3->Col[0], nnz3, st);
     const int sms = sm_count();
     auto grid = [&](int64_t work) { return (int)std::max<int64_t>(1, std::min<int64_t>((work + kThreads - 1) / kThreads, (int64_t)sms * 8)); };
+    // a block per column of the result, its threads over the rows
+    auto grid2 = [&](int rows, int cols) { return dim3((unsigned)grid(rows), (unsigned)std::max(1, std::min(cols, 65535))); };
+    DevBuf<Span> s1(std::max(row_m1, 1)), s2(std::max(row_m2, 1)), s3(std::max(col_m3, 1));
+    DevBuf<int> odd(3);   // a non-finite value in M2 / in W / in M1 or M3 (not needed)
+    DG_CUDA(cudaMemsetAsync(odd.get(), 0, sizeof(int) * 3, st));
     // W = M2 M3 (dense, by columns), then its CCS
     DevBuf<double> D3((size_t)row_m3 * col_m3), Wd((size_t)row_m2 * col_m3);
     DG_CUDA(cudaMemsetAsync(D3.get(), 0, sizeof(double) * D3.n, st));
-    k_scatter_cols<<<grid(col_m3), kThreads, 0, st>>>(col_m3, d_p3.get(), d_r3.get(), d_v3.get(), row_m3, D3.get());
+    k_lines<<<grid((int64_t)col_m3 * 32), kThreads, 0, st>>>(col_m3, d_p3.get(), d_r3.get(), d_v3.get(), s3.get(), D3.get(), row_m3, 1,
+                                                             odd.get() + 2);
     count_launch();
-    k_rows_times_dense<<<grid((int64_t)row_m2 * col_m3), kThreads, 0, st>>>(row_m2, col_m3, d_p2.get(), d_c2.get(), d_v2.get(), D3.get(),
-                                                                          row_m3, Wd.get());
+    k_lines<<<grid((int64_t)row_m2 * 32), kThreads, 0, st>>>(row_m2, d_p2.get(), d_c2.get(), d_v2.get(), s2.get(), nullptr, 0, 0,
+                                                             odd.get());
+    count_launch();
+    k_rows_times_dense<<<grid2(row_m2, col_m3), kThreads, 0, st>>>(row_m2, col_m3, d_p2.get(), d_c2.get(), d_v2.get(), s2.get(), s3.get(),
+                                                                   odd.get(), D3.get(), row_m3, Wd.get(), odd.get() + 1);
     count_launch();
     DevBuf<int64_t> wcnt(col_m3), woff(col_m3);
     k_compact_lines<<<grid((int64_t)col_m3 * kThreads), kThreads, 0, st>>>(col_m3, row_m2, Wd.get(), row_m2, 1, 0, wcnt.get(), nullptr,
@@ -203,10 +289,11 @@ void crs_crs_ccs(CRS1 *M1, CRS1 *M2, CCS1 *M3, CRS1 *Out, CCS1 *Work, double *Wo
     // Out = M1 W (dense, by columns), then its CRS
     DevBuf<double> D1((size_t)row_m2 * row_m1), Od((size_t)row_m1 * col_m3);
     DG_CUDA(cudaMemsetAsync(D1.get(), 0, sizeof(double) * D1.n, st));
-    k_scatter_rows_t<<<grid(row_m1), kThreads, 0, st>>>(row_m1, d_p1.get(), d_c1.get(), d_v1.get(), row_m1, D1.get());
+    k_lines<<<grid((int64_t)row_m1 * 32), kThreads, 0, st>>>(row_m1, d_p1.get(), d_c1.get(), d_v1.get(), s1.get(), D1.get(), 1, row_m1,
+                                                             odd.get() + 2);
     count_launch();
-    k_dense_times_cols<<<grid((int64_t)row_m1 * col_m3), kThreads, 0, st>>>(row_m1, col_m3, d_wo.get(), Wr.get(), Wv.get(), D1.get(),
-                                                                          Od.get());
+    k_dense_times_cols<<<grid2(row_m1, col_m3), kThreads, 0, st>>>(row_m1, col_m3, d_wo.get(), Wr.get(), Wv.get(), s1.get(),
+                                                                   odd.get() + 1, D1.get(), Od.get());
     count_launch();
     DevBuf<int64_t> ocnt(row_m1);
     k_compact_lines<<<grid((int64_t)row_m1 * kThreads), kThreads, 0, st>>>(row_m1, col_m3, Od.get(), 1, row_m1, 0, ocnt.get(), nullptr,
