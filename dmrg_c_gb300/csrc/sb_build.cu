@@ -7,14 +7,23 @@
 // absent; the row keeps (0 <= col <= row and |v| > 1e-15) or col == row, and
 // SORT_COLUMN_CRS1 orders the columns.
 //
-// GB300 form: one warp per row.  The lanes enumerate the row's generated elements term by
-// term (element k of a two-operator term is op1 entry k / c2 times op2 entry k % c2, the
-// reference's loop order), compute value and target column in parallel, and compact the
-// accepted ones (|v| > 1e-15, target in the sector) into shared memory with key
-// (column << 22 | generation index).  A bitonic sort of the keys puts every column's
-// contributions together in generation order, so summing each run left to right reproduces
-// the reference's accumulation bit for bit; the sorted runs are already in column order.
-// Pass 1 counts kept entries per row, a scan gives the row offsets, pass 2 fills.
+// GB300 form: one warp per row.  The lanes read the row's term list 32 terms at a time (a lane
+// per term: operator rows, fermion sign, target offsets), then walk the generated elements of all
+// of them together (element k of a two-operator term is op1 entry k / c2 times op2 entry k % c2,
+// the reference's loop order), compute value and target column in parallel, and compact the
+// accepted ones (|v| > 1e-15, target in the sector and in the lower triangle, the only ones the
+// row can keep) into shared memory with key (column << 22 | generation position).  A bitonic sort
+// of the keys puts every column's contributions together in generation order, so summing each run
+// left to right reproduces the reference's accumulation bit for bit; the sorted runs are already in
+// column order.  The rows are generated once, into a scratch with room for every row's generated
+// elements, and compacted behind a scan of the kept counts; where that scratch would be too large
+// a count pass and a fill pass generate them twice.
+//
+// Measured on the Hubbard m=512 superblock of a DMRG run (238 k rows, 325 generated elements a row,
+// 28.2 M kept): two passes of 8.96 ms with every term walked by itself (22 terms of ~15 elements:
+// most lanes idle, a chain of four dependent loads a term), the upper triangle sorted along and 12
+// warps a SM (16 KB of buffer a warp, sized by the operators' widest rows instead of the rows
+// themselves).  Term list to solver operator and first product: 22.3 -> 6.4 ms.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -46,76 +55,150 @@ struct SbDev {
   double zero;
 };
 
-constexpr int kGenBits = 22;      // generation index bits of a sort key
+constexpr int kGenBits = 22;      // generation position bits of a sort key
+constexpr int kSbWarps = 4;       // warps a block, at most
+constexpr int kSbTerms = 32;      // terms a warp holds at once: a lane each
+constexpr size_t kSbScratchBytes = size_t(2) << 30;   // scratch of the single-pass build, at most
 
-__global__ void k_sb_rows(SbDev m, int cap, long long *__restrict__ counts, const int64_t *__restrict__ row,
-                          int *__restrict__ col, double *__restrict__ val, int *err) {
-  extern __shared__ unsigned char smem[];
-  const int warps = blockDim.x >> 5;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// A term of the row at hand.
+struct SbRowTerm {
+  int64_t sup, m1, m2;            // target position: sup + col1 * m1 + col2 * m2
+  double sc;                      // sign * coefficient
+  int e1, e2, c2, first;          // first elements of op1 and op2 (e2 < 0: one operator), op2's
+                                  // row length, first generated element of the term
+};
+
+// bound[b] = generated elements of row b; *most = the largest.
+__global__ void __launch_bounds__(kThreads) k_sb_bounds(SbDev m, long long *__restrict__ bound, int *__restrict__ most) {
+  int mx = 0;
+  for (long b = (long)blockIdx.x * blockDim.x + threadIdx.x; b < m.n; b += (long)gridDim.x * blockDim.x) {
+    long long g = 0;
+    for (int t = 0; t < m.n_terms; ++t) {
+      const SbTermDev T = m.terms[t];
+      if (fabs(T.coef) < m.zero) continue;
+      const int64_t *r1 = m.op_row + m.op_row_base[T.op1] + m.st[T.pos1][b];
+      long long c = r1[1] - r1[0];
+      if (T.pos2 >= 0) {
+        const int64_t *r2 = m.op_row + m.op_row_base[T.op2] + m.st[T.pos2][b];
+        c *= r2[1] - r2[0];
+      }
+      g += c;
+    }
+    bound[b] = g + 1;   // + the zero diagonal
+    mx = max(mx, (int)g);
+  }
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if ((threadIdx.x & 31) == 0) atomicMax(most, mx);
+}
+
+// Rows of the lower triangle.  soff set: row b's kept elements to col/val[soff[b] ...] (room for its
+// bound), their number to counts[b]; else row set: the fill pass, to col/val[row[b] ...]; else the
+// count pass.  err: 1 buffer overflow, 2 fill pass and count pass disagree.
+__global__ void __launch_bounds__(kSbWarps * 32) k_sb_rows(SbDev m, int cap, const int64_t *__restrict__ soff,
+                                                           long long *__restrict__ counts, const int64_t *__restrict__ row,
+                                                           int *__restrict__ col, double *__restrict__ val, int *err) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ SbRowTerm s_term[kSbWarps][kSbTerms];
+  const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint64_t *keys = reinterpret_cast<uint64_t *>(smem) + (size_t)warp * cap;
   double *vals = reinterpret_cast<double *>(smem + (size_t)warps * cap * sizeof(uint64_t)) + (size_t)warp * cap;
+  SbRowTerm *const rt = s_term[warp];
   const unsigned FULL = 0xffffffffu;
   const unsigned lt = (1u << lane) - 1u;
+  const int64_t mult[4] = {(int64_t)m.d * m.dim_RR * m.d, (int64_t)m.dim_RR * m.d, m.d, 1};
   for (long b = (long)blockIdx.x * warps + warp; b < m.n; b += (long)gridDim.x * warps) {
     int st[4];
 #pragma unroll
     for (int p = 0; p < 4; ++p) st[p] = m.st[p][b];
+    const int64_t sup0 = st[0] * mult[0] + st[1] * mult[1] + st[2] * mult[2] + st[3];
     int nitems = 0;
-    long gbase = 0;
-    for (int t = 0; t < m.n_terms; ++t) {
-      const SbTermDev T = m.terms[t];
-      if (fabs(T.coef) < m.zero) continue;
-      const int64_t *r1 = m.op_row + m.op_row_base[T.op1];
-      const int s1 = st[T.pos1];
-      const int a1 = (int)r1[s1], c1 = (int)(r1[s1 + 1] - r1[s1]);
-      int a2 = 0, c2 = 1;
-      if (T.pos2 >= 0) {
-        const int64_t *r2 = m.op_row + m.op_row_base[T.op2];
-        const int s2 = st[T.pos2];
-        a2 = (int)r2[s2];
-        c2 = (int)(r2[s2 + 1] - r2[s2]);
-      }
-      const long total = (long)c1 * c2;
-      int sign = 1;
-      if (T.sign_mask) {
-        int ne = 0;
+    for (int t0 = 0; t0 < m.n_terms; t0 += kSbTerms) {
+      // the terms' operator rows, signs and target offsets: a lane per term
+      const int nt = min(kSbTerms, m.n_terms - t0);
+      int mine = 0;
+      SbRowTerm R{};
+      if (lane < nt) {
+        const SbTermDev T = m.terms[t0 + lane];
+        if (!(fabs(T.coef) < m.zero)) {
+          int s1 = 0, s2 = 0;
 #pragma unroll
-        for (int p = 0; p < 4; ++p)
-          if (T.sign_mask & (1 << p)) ne += m.ele[p][st[p]];
-        sign = (ne % 2 == 0) ? T.sign_even : -T.sign_even;
+          for (int p = 0; p < 4; ++p) {
+            if (T.pos1 == p) {
+              s1 = st[p];
+              R.m1 = mult[p];
+            }
+            if (T.pos2 == p) {
+              s2 = st[p];
+              R.m2 = mult[p];
+            }
+          }
+          const int64_t *r1 = m.op_row + m.op_row_base[T.op1] + s1;
+          R.e1 = m.op_first[T.op1] + (int)r1[0];
+          mine = (int)(r1[1] - r1[0]);
+          R.sup = sup0 - s1 * R.m1 - s2 * R.m2;
+          R.c2 = 1;
+          R.e2 = -1;
+          R.sc = T.coef;
+          if (T.pos2 >= 0) {
+            const int64_t *r2 = m.op_row + m.op_row_base[T.op2] + s2;
+            R.e2 = m.op_first[T.op2] + (int)r2[0];
+            R.c2 = (int)(r2[1] - r2[0]);
+            mine *= R.c2;
+            int sign = 1;
+            if (T.sign_mask) {
+              int ne = 0;
+#pragma unroll
+              for (int p = 0; p < 4; ++p)
+                if (T.sign_mask & (1 << p)) ne += m.ele[p][st[p]];
+              sign = (ne % 2 == 0) ? T.sign_even : -T.sign_even;
+            }
+            R.sc = __dmul_rn((double)sign, T.coef);
+          }
+        }
       }
-      const double sc = __dmul_rn((double)sign, T.coef);
-      for (long k0 = 0; k0 < total; k0 += 32) {
-        const long k = k0 + lane;
+      int incl = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o) incl += v;
+      }
+      const int total = __shfl_sync(FULL, incl, 31);
+      R.first = incl - mine;
+      __syncwarp();   // the previous terms' readers are done
+      rt[lane] = R;   // lanes past nt: first = total, never selected
+      __syncwarp();
+      // the generated elements of these terms, 32 at a time
+      for (int k0 = 0; k0 < total; k0 += 32) {
+        const int k = k0 + lane;
         bool acc = false;
         int64_t tgt = -1;
         double v = 0.0;
         if (k < total) {
-          int ns[4] = {st[0], st[1], st[2], st[3]};
-          const int i = (int)(k / c2), j = (int)(k % c2);
-          const int e1 = m.op_first[T.op1] + a1 + i;
-          ns[T.pos1] = m.op_col[e1];
-          if (T.pos2 >= 0) {
-            const int e2 = m.op_first[T.op2] + a2 + j;
-            ns[T.pos2] = m.op_col[e2];
-            v = __dmul_rn(__dmul_rn(sc, m.op_val[e1]), m.op_val[e2]);
-          } else {
-            v = __dmul_rn(T.coef, m.op_val[e1]);
+          int lo = 0;   // the last term whose first element is at or before k (empty terms: the last of equals)
+#pragma unroll
+          for (int step = kSbTerms / 2; step > 0; step >>= 1)
+            if (rt[lo + step].first <= k) lo += step;
+          const SbRowTerm &T = rt[lo];
+          const int r = k - T.first;
+          const int i = T.c2 == 1 ? r : r / T.c2, j = T.c2 == 1 ? 0 : r - i * T.c2;
+          const int e1 = T.e1 + i;
+          int64_t sup = T.sup + m.op_col[e1] * T.m1;
+          v = __dmul_rn(T.sc, m.op_val[e1]);
+          if (T.e2 >= 0) {
+            sup += m.op_col[T.e2 + j] * T.m2;
+            v = __dmul_rn(v, m.op_val[T.e2 + j]);
           }
-          const int64_t sup = (((int64_t)ns[0] * m.d + ns[1]) * m.dim_RR + ns[2]) * m.d + ns[3];
           tgt = m.inv[sup];
-          acc = fabs(v) > m.zero && tgt >= 0;
+          acc = tgt >= 0 && tgt <= b && fabs(v) > m.zero;
         }
         const unsigned bal = __ballot_sync(FULL, acc);
         const int pos = nitems + __popc(bal & lt);
         if (acc && pos < cap) {
-          keys[pos] = ((uint64_t)tgt << kGenBits) | (uint64_t)(gbase + k);
+          keys[pos] = ((uint64_t)tgt << kGenBits) | (uint64_t)pos;
           vals[pos] = v;
         }
         nitems += __popc(bal);
       }
-      gbase += total;
     }
     if (nitems > cap) {
       if (lane == 0) {
@@ -124,33 +207,29 @@ __global__ void k_sb_rows(SbDev m, int cap, long long *__restrict__ counts, cons
       }
       continue;
     }
-    // bitonic sort of the keys (vals follow), padded to a power of two
+    // bitonic sort of the keys, padded to a power of two (the values stay where they are)
     int P = 1;
     while (P < nitems) P <<= 1;
     for (int p = nitems + lane; p < P; p += 32) keys[p] = ~0ull;
     __syncwarp();
     for (int kk = 2; kk <= P; kk <<= 1) {
       for (int j = kk >> 1; j > 0; j >>= 1) {
-        for (int i = lane; i < P; i += 32) {
-          const int ixj = i ^ j;
-          if (ixj > i) {
-            const bool up = (i & kk) == 0;
-            const uint64_t ki = keys[i], kj = keys[ixj];
-            if ((ki > kj) == up) {
-              keys[i] = kj;
-              keys[ixj] = ki;
-              const double vi = vals[i];
-              vals[i] = vals[ixj];
-              vals[ixj] = vi;
-            }
+        for (int i = lane; i < P / 2; i += 32) {
+          const int lo = ((i & ~(j - 1)) << 1) | (i & (j - 1)), hi = lo | j;   // the pair's lower index has bit j clear
+          const uint64_t ka = keys[lo], kb = keys[hi];
+          if ((ka > kb) == ((lo & kk) == 0)) {
+            keys[lo] = kb;
+            keys[hi] = ka;
           }
         }
         __syncwarp();
       }
     }
-    // runs of equal column, summed in generation order; keep the lower triangle + diagonal
-    const int64_t start = row ? row[b] : 0, end = row ? row[b + 1] : 0;
-    long long kept = 0;
+    // runs of equal column, summed in generation order
+    const int64_t start = soff ? soff[b] : (row ? row[b] : 0), end = soff ? soff[b + 1] : (row ? row[b + 1] : 0);
+    const bool write = soff || row;
+    const uint64_t gen = (1ull << kGenBits) - 1;
+    int kept = 0;
     bool have_diag = false;
     for (int c0 = 0; c0 < nitems; c0 += 32) {
       const int p = c0 + lane;
@@ -158,17 +237,18 @@ __global__ void k_sb_rows(SbDev m, int cap, long long *__restrict__ counts, cons
       int64_t t = -1;
       double sum = 0.0;
       if (p < nitems) {
-        t = (int64_t)(keys[p] >> kGenBits);
+        const uint64_t key = keys[p];
+        t = (int64_t)(key >> kGenBits);
         const bool head = (p == 0) || ((int64_t)(keys[p - 1] >> kGenBits) != t);
         if (head) {
-          sum = vals[p];
-          for (int q = p + 1; q < nitems && (int64_t)(keys[q] >> kGenBits) == t; ++q) sum = __dadd_rn(sum, vals[q]);
-          keep = (t <= b && fabs(sum) > m.zero) || t == b;
+          sum = vals[key & gen];
+          for (int q = p + 1; q < nitems && (int64_t)(keys[q] >> kGenBits) == t; ++q) sum = __dadd_rn(sum, vals[keys[q] & gen]);
+          keep = fabs(sum) > m.zero || t == b;
           diag = t == b;
         }
       }
       const unsigned kb = __ballot_sync(FULL, keep);
-      if (row && keep) {
+      if (write && keep) {
         const int64_t pos = start + kept + __popc(kb & lt);
         if (pos < end) {
           col[pos] = (int)t;
@@ -179,7 +259,7 @@ __global__ void k_sb_rows(SbDev m, int cap, long long *__restrict__ counts, cons
       have_diag = have_diag || __any_sync(FULL, diag);
     }
     if (!have_diag) {   // DMRG_MAKE_ELEM_ZERO_LLLRRRRL: a zero diagonal, the row's largest column
-      if (row && lane == 0 && start + kept < end) {
+      if (write && lane == 0 && start + kept < end) {
         col[start + kept] = (int)b;
         val[start + kept] = 0.0;
       }
@@ -187,9 +267,25 @@ __global__ void k_sb_rows(SbDev m, int cap, long long *__restrict__ counts, cons
     }
     if (lane == 0) {
       if (counts) counts[b] = kept;
-      if (row && start + kept != end) atomicExch(err, 2);
+      if (row && !soff && start + kept != end) atomicExch(err, 2);
     }
     __syncwarp();
+  }
+}
+
+// Row b's kept elements from the scratch (at soff[b]) to col/val[row[b] ...].  One warp a row.
+__global__ void __launch_bounds__(kThreads) k_sb_compact(int n, const int64_t *__restrict__ soff, const int64_t *__restrict__ row,
+                                                        const int *__restrict__ scol, const double *__restrict__ sval,
+                                                        int *__restrict__ col, double *__restrict__ val) {
+  const int lane = threadIdx.x & 31;
+  const long nw = (long)gridDim.x * kWarps;
+  for (long b = blockIdx.x * (long)kWarps + (threadIdx.x >> 5); b < n; b += nw) {
+    const int64_t src = soff[b], dst = row[b];
+    const int cnt = (int)(row[b + 1] - dst);
+    for (int k = lane; k < cnt; k += 32) {
+      col[dst + k] = scol[src + k];
+      val[dst + k] = sval[src + k];
+    }
   }
 }
 
@@ -273,8 +369,6 @@ dg_sb *sb_build(const dg_sb_model *m, const SbBasisView *bv) {
   DG_REQUIRE(gen_bound < (1L << kGenBits), DG_ERR_ARG, "a row can generate %ld elements (limit %ld)", gen_bound, 1L << kGenBits);
   const int cap_need = (int)std::min<long>(gen_bound + 1, 1L << 30);
   DG_REQUIRE(cap_need <= 4096, DG_ERR_ARG, "a row can keep %d elements; at most 4096 are supported", cap_need);
-  int cap = 32;
-  while (cap < cap_need) cap <<= 1;
 
   cudaStream_t st = stream();
   // device copies
@@ -352,18 +446,49 @@ dg_sb *sb_build(const dg_sb_model *m, const SbBasisView *bv) {
   dev.zero = std::pow(10.0, -15.0);
   DG_CUDA(cudaMemsetAsync(err.get(), 0, sizeof(int), st));
 
-  // launch shape: warps per block bounded by 96 KB of shared memory
-  const size_t per_warp = (size_t)cap * (sizeof(uint64_t) + sizeof(double));
-  const int warps = (int)std::max<size_t>(1, std::min<size_t>(4, (96u << 10) / per_warp));
-  const size_t smem = per_warp * warps;
-  DG_CUDA(cudaFuncSetAttribute(k_sb_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const long blocks = std::max(1L, std::min<long>((n + warps - 1) / warps, (long)sm_count() * 32));
-
   dg_sb *s = new dg_sb();
   try {
     s->n = n;
     DevBuf<long long> counts(n), tmp((n + kScanTile - 1) / kScanTile + 2);
-    k_sb_rows<<<(int)blocks, warps * 32, smem, st>>>(dev, cap, counts.get(), nullptr, nullptr, nullptr, err.get()); ::dg::count_launch();
+    DevBuf<int64_t> soff(n + 1);
+    DevBuf<int> most(1);
+    // every row's generated elements: the scratch offsets, and the largest row, which sizes a warp's
+    // buffer (the operators' widest rows seldom meet in one superblock row: 490 against a bound of
+    // 960 on the Hubbard m=512 superblock, which doubles the warps a SM holds)
+    DG_CUDA(cudaMemsetAsync(most.get(), 0, sizeof(int), st));
+    k_sb_bounds<<<(int)std::max(1L, std::min<long>((n + kThreads - 1) / kThreads, (long)sm_count() * 8)), kThreads, 0, st>>>(
+        dev, counts.get(), most.get()); ::dg::count_launch();
+    DG_CUDA(cudaGetLastError());
+    exclusive_scan(counts.get(), n, soff.get(), tmp.get(), st);
+    int64_t bound = 0;
+    int hmost = 0;
+    DG_CUDA(cudaMemcpyAsync(&bound, soff.get() + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    DG_CUDA(cudaMemcpyAsync(&hmost, most.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
+    DG_CUDA(cudaStreamSynchronize(st));
+    int cap = 32;
+    while (cap < hmost) cap <<= 1;
+    // warps a block bounded by 192 KB of shared memory (cap <= 4096: three warps at least)
+    const size_t per_warp = (size_t)cap * (sizeof(uint64_t) + sizeof(double));
+    const int warps = (int)std::min<size_t>(kSbWarps, (192u << 10) / per_warp);
+    const size_t smem = per_warp * warps;
+    DG_CUDA(cudaFuncSetAttribute(k_sb_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const long blocks = std::max(1L, std::min<long>((n + warps - 1) / warps, (long)sm_count() * 32));
+    DevBuf<int> scol;
+    DevBuf<double> sval;
+    bool single = (size_t)bound * (sizeof(int) + sizeof(double)) <= kSbScratchBytes;
+    if (single) {
+      try {
+        scol.alloc(bound);
+        sval.alloc(bound);
+      } catch (const Error &e) {   // no room for the scratch: the two passes need none
+        if (e.code != DG_ERR_NOMEM) throw;
+        cudaGetLastError();
+        scol.release();
+        single = false;
+      }
+    }
+    k_sb_rows<<<(int)blocks, warps * 32, smem, st>>>(dev, cap, single ? soff.get() : (const int64_t *)nullptr, counts.get(), nullptr,
+                                                        scol.get(), sval.get(), err.get()); ::dg::count_launch();
     DG_CUDA(cudaGetLastError());
     s->row.alloc(n + 1);
     exclusive_scan(counts.get(), n, s->row.get(), tmp.get(), st);
@@ -376,11 +501,19 @@ dg_sb *sb_build(const dg_sb_model *m, const SbBasisView *bv) {
     s->nnz = total;
     s->col.alloc(total);
     s->val.alloc(total);
-    k_sb_rows<<<(int)blocks, warps * 32, smem, st>>>(dev, cap, nullptr, s->row.get(), s->col.get(), s->val.get(), err.get()); ::dg::count_launch();
-    DG_CUDA(cudaGetLastError());
-    DG_CUDA(cudaMemcpyAsync(&herr, err.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
-    DG_CUDA(cudaStreamSynchronize(st));
-    DG_REQUIRE(herr == 0, DG_ERR_INTERNAL, "superblock fill pass disagreed with the count pass (%d)", herr);
+    if (single) {
+      k_sb_compact<<<(int)std::max(1L, std::min<long>((n + kWarps - 1) / kWarps, (long)sm_count() * 16)), kThreads, 0, st>>>(
+          n, soff.get(), s->row.get(), scol.get(), sval.get(), s->col.get(), s->val.get()); ::dg::count_launch();
+      DG_CUDA(cudaGetLastError());
+      DG_CUDA(cudaStreamSynchronize(st));
+    } else {
+      k_sb_rows<<<(int)blocks, warps * 32, smem, st>>>(dev, cap, nullptr, nullptr, s->row.get(), s->col.get(), s->val.get(),
+                                                          err.get()); ::dg::count_launch();
+      DG_CUDA(cudaGetLastError());
+      DG_CUDA(cudaMemcpyAsync(&herr, err.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
+      DG_CUDA(cudaStreamSynchronize(st));
+      DG_REQUIRE(herr == 0, DG_ERR_INTERNAL, "superblock fill pass disagreed with the count pass (%d)", herr);
+    }
   } catch (...) {
     delete s;
     throw;
