@@ -994,7 +994,7 @@ int batch_post(const BatchDone &d, const dg_solver_params &p, double *eigvec, dg
       throw Error{d.status};
     }
     const CrsLauncher op{d.m};
-    Workspace ws(d.m->n, op.grid(), st);
+    Workspace ws(d.m->n, std::max(op.grid(), op.grid32()), st);
     if (p.mixed) {
       RefineResult R = refine_core(op, p.ii_acc, p.ii_max_step + 1, p.cg_max_step, d.psi, ws);
       info->eig_val = R.eig_val;

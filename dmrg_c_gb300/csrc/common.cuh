@@ -271,6 +271,42 @@ __device__ __forceinline__ void block_partial(double v, double *partials) {
   if (threadIdx.x == 0) partials[blockIdx.x] = b;
 }
 
+// N sums over a block of T threads, valid in warp 0: the values transposed through shared memory,
+// each lane of warp 0 adding its column as a pairwise tree, then a shuffle tree.  The N trees overlap:
+// an FP64 add has a latency of ~60 cycles on GB300 and a tree is a chain of eight or nine.
+template <int T, int N>
+__device__ __forceinline__ void block_sums(double (&v)[N]) {
+  static_assert(T == 256 || T == 512, "column trees below are written for 8 or 16 warps");
+  __shared__ double sm[N][T];
+  __syncthreads();   // an earlier call's readers are done with sm
+#pragma unroll
+  for (int k = 0; k < N; ++k) sm[k][threadIdx.x] = v[k];
+  __syncthreads();
+  if (threadIdx.x < 32) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      double h[T / 64];
+#pragma unroll
+      for (int j = 0; j < T / 64; ++j) h[j] = sm[k][threadIdx.x + 64 * j] + sm[k][threadIdx.x + 64 * j + 32];
+#pragma unroll
+      for (int w = T / 128; w > 0; w >>= 1)
+#pragma unroll
+        for (int j = 0; j < w; ++j) h[j] = h[2 * j] + h[2 * j + 1];
+      v[k] = h[0];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int k = 0; k < N; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+  }
+}
+// Per-thread share of count partials written by the previous kernel.
+__device__ __forceinline__ double partials_share(const double *partials, int count) {
+  double s = 0.0;
+  for (int i = threadIdx.x; i < count; i += blockDim.x) s += __ldcg(partials + i);
+  return s;
+}
+
 // Sum of count partials written by the previous kernel; valid in every thread.
 __device__ __forceinline__ double sum_partials(const double *partials, int count) {
   __shared__ double s_total;

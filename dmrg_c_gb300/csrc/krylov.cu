@@ -27,76 +27,6 @@ __global__ void k_random_start(double *x, int n, unsigned long long seed) {
   }
 }
 
-__global__ void __launch_bounds__(kThreads) k_cg_update(int n, const double *__restrict__ p, const double *__restrict__ y,
-                                                       double *__restrict__ x, double *__restrict__ r, const Scalars *S, int it,
-                                                       const double *pp, int pcount, double *up) {
-  pdl_wait();
-  if (*((volatile const int *)&S->done)) return;
-  // first element's operands in flight before the partial sums (see k_lz_update)
-  const int i0 = blockIdx.x * kThreads + threadIdx.x, stride = gridDim.x * kThreads;
-  double x0 = 0.0, p0 = 0.0, r0 = 0.0, y0 = 0.0;
-  if (i0 < n) {
-    x0 = x[i0];
-    p0 = p[i0];
-    r0 = r[i0];
-    y0 = y[i0];
-  }
-  __shared__ double s_a;
-  const double py = sum_partials(pp, pcount);
-  if (threadIdx.x == 0) s_a = S->rrs[it & 1] / py;   // one division per block
-  __syncthreads();
-  const double a = s_a;
-  double acc = 0.0;
-  auto step = [&](int i, double xi, double pi, double ri, double yi) {
-    x[i] = xi + a * pi;
-    const double rn = ri - a * yi;
-    r[i] = rn;
-    acc += rn * rn;
-  };
-  if (i0 < n) step(i0, x0, p0, r0, y0);
-  for (int i = i0 + stride; i < n; i += stride) step(i, x[i], p[i], r[i], y[i]);
-  pdl_trigger();
-  block_partial(acc, up);
-}
-
-__global__ void __launch_bounds__(kThreads) k_cg_direction(int n, const double *__restrict__ r, double *__restrict__ p, Scalars *S,
-                                                          int it, int max_step, double acc_thr, const double *up, int ucount,
-                                                          Progress *prog) {
-  pdl_wait();
-  if (*((volatile const int *)&S->done)) return;
-  // first element's operands in flight before the partial sums (see k_lz_update)
-  const int i0 = blockIdx.x * kThreads + threadIdx.x, stride = gridDim.x * kThreads;
-  double r0 = 0.0, p0 = 0.0;
-  if (i0 < n) {
-    r0 = r[i0];
-    p0 = p[i0];
-  }
-  __shared__ double s_b;
-  const double t = sum_partials(up, ucount);
-  const bool converged = t < acc_thr, last = it >= max_step - 1;
-  if (threadIdx.x == 0) {
-    if (blockIdx.x == 0) {
-      if (converged) {
-        S->done = 1;
-        S->iters = it;
-      } else if (last) {
-        S->done = 2;
-        S->iters = max_step;
-      }
-      S->rrs[(it + 1) & 1] = t;   // the other slot: this kernel's blocks read rrs[it & 1]
-      prog->done = S->done;
-      prog->stamp = it;
-    }
-    s_b = t / S->rrs[it & 1];
-  }
-  __syncthreads();
-  if (converged || last) return;   // the same decision in every block
-  const double b = s_b;
-  if (i0 < n) p[i0] = r0 + b * p0;
-  for (int i = i0 + stride; i < n; i += stride) p[i] = r[i] + b * p[i];
-  pdl_trigger();
-}
-
 // V2 = Temp - delta V1 - gamma0 V0, gamma1 = ||V2||, Givens rotation, eta update and the
 // convergence test |eta| < acc (sml/MINIMUM_RESIDUAL_SYM.c:62-90).
 __global__ void __launch_bounds__(kThreads) k_mr_lanczos(int n, const double *__restrict__ temp, const double *__restrict__ v1n,

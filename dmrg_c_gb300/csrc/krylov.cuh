@@ -56,6 +56,20 @@ struct Progress {
   volatile int done;
 };
 
+// Launch shape of the step kernels (k_lz_step, k_cg_update, k_cg_direction).  Every block sums the product's partials (up to ~1,900 a
+// sum) before its elements, and on GB300 a warp-wide FP64 add holds an SM's FP64 pipe for ~19
+// cycles: with four blocks a SM those sums were most of the kernels' time at 238 k elements (9.6 us
+// for 2 us of traffic).  So large vectors get one block of 512 threads a SM; small ones, where the
+// elements' own FP64 work counts, one thread an element.
+constexpr int kStepAhead = 2;   // elements a thread loads before the partial sums
+inline int update_threads(long n) { return n > (long)sm_count() * 2 * kThreads ? 512 : kThreads; }
+inline int update_grid(long n) {
+  const int t = update_threads(n);
+  // two blocks a SM again where the vectors' traffic outweighs the sums (XXZ L=22, 705 k states)
+  const int per_sm = t == kThreads || n > (long)sm_count() * 2048 ? 2 : 1;
+  return (int)std::max(1L, std::min((n + t - 1) / t, (long)sm_count() * per_sm));
+}
+
 // ---------------------------------------------------------------------------------
 // Per-solve workspace.
 // ---------------------------------------------------------------------------------
@@ -63,12 +77,15 @@ struct Workspace {
   cudaStream_t st;
   int n;
   int vgrid;
+  int uthreads, ugrid;   // launch shape of the step kernels
   DevBuf<double> partials, partials2, partials3;   // 2, 3: more slots for consumer-finished reductions
   DevBuf<unsigned> ticket;
   DevBuf<Scalars> sc;
   Mapped<Progress> prog;
   explicit Workspace(int n_, int max_grid, cudaStream_t s) : st(s), n(n_) {
     vgrid = vector_grid(n_);
+    uthreads = update_threads(n_);
+    ugrid = update_grid(n_);
     int g = max_grid > vgrid ? max_grid : vgrid;
     partials.alloc(g);
     partials2.alloc(g);
@@ -207,51 +224,99 @@ struct EpiLanczos {
   }
 };
 
-// Step b: D[b] = <y, v_b> summed from the product's pcount block partials (block 0 records it
-// and its host mirror), or, with pcount 0, as the product's last block recorded it;
-// w = y - D[b] v_b - O[b] v_{b-1} (sml/LANCZOS_SYM.c:121-125, 240-243).
-// <w,w>: with r2 null, block partials into out.partials for the next product to sum; else the
-// last block forms the Norm2 *r2.
+// Product of a Lanczos step on the unnormalised vector: y = H w, block partials of <y, w>.  Nothing in
+// it waits for ||w||: the step kernel forms it beside <y, w>.
+struct EpiLzRaw {
+  static constexpr bool kReduce = true;
+  static constexpr bool kDeferred = true;
+  double *y;
+  __device__ void row(int i, double xi, double yi, double &acc) const {
+    y[i] = yi;
+    acc += yi * xi;
+  }
+  __device__ void finalize(double) const {}
+};
+
+// Step b on w_b (unnormalised; w_0 normalised) and y = H w_b: beta_b = ||w_b|| (b > 0: from the previous
+// step's vcount partials in rp; O[b] = beta_b, 0 for b = 0), v_b = w_b / beta_b into v, alpha_b =
+// <y, w_b> / beta_b^2 (the product's pcount partials in pp; D[b]), then
+// w_{b+1} = y / beta_b - alpha_b v_b - beta_b v_{b-1} (sml/LANCZOS_SYM.c:121-143, 240-243) into w, block
+// partials of <w,w> into wp.  Block 0 records D, O and their host mirrors.
+template <int T>
+__global__ void __launch_bounds__(T) k_lz_step(int n, const double *__restrict__ y, double *__restrict__ w, double *__restrict__ v,
+                                              const double *__restrict__ vprev, double *D, double *O, double *hD, double *hO, int b,
+                                              const double *pp, int pcount, const double *rp, int rcount, double *wp) {
+  __shared__ double s_sc[3];
+  pdl_wait();
+  // the first elements' operands are loaded before the partial sums, so that the L2 round trips overlap
+  const int i0 = blockIdx.x * T + threadIdx.x, stride = gridDim.x * T;
+  constexpr int U = kStepAhead;
+  double y0[U], w0[U], p0[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int i = i0 + u * stride;
+    const bool in = i < n;
+    y0[u] = in ? y[i] : 0.0;
+    w0[u] = in ? w[i] : 0.0;
+    p0[u] = in && b > 0 ? vprev[i] : 0.0;
+  }
+  {
+    double t[2] = {partials_share(pp, pcount), b > 0 ? partials_share(rp, rcount) : 0.0};
+    block_sums<T, 2>(t);
+    if (threadIdx.x == 0) {
+      const double o = b > 0 ? sqrt(t[1]) : 0.0, sc = b > 0 ? 1.0 / o : 1.0;
+      const double d = t[0] * sc * sc;
+      s_sc[0] = d;
+      s_sc[1] = o;
+      s_sc[2] = sc;
+      if (blockIdx.x == 0) {
+        D[b] = d;
+        O[b] = o;
+        hD[b] = d;
+        hO[b] = o;
+      }
+    }
+  }
+  __syncthreads();
+  const double d = s_sc[0], o = s_sc[1], sc = s_sc[2];
+  double acc = 0.0;
+  auto step = [&](int i, double yi, double wi, double pi) {
+    const double vi = b > 0 ? wi * sc : wi;
+    if (b > 0) yi *= sc;
+    double r = yi - d * vi;
+    if (b > 0) r = r - o * pi;
+    v[i] = vi;
+    w[i] = r;
+    acc += r * r;
+  };
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (i0 + u * stride < n) step(i0 + u * stride, y0[u], w0[u], p0[u]);
+#pragma unroll 2
+  for (int i = i0 + U * stride; i < n; i += stride) step(i, y[i], w[i], b > 0 ? vprev[i] : 0.0);
+  pdl_trigger();
+  double t[1] = {acc};
+  block_sums<T, 1>(t);
+  if (threadIdx.x == 0) wp[blockIdx.x] = t[0];
+}
+
+// Step b of the dense path: w = y - D[b] v_b - O[b] v_{b-1} (sml/LANCZOS_SYM.c:121-125, 240-243); the last
+// block forms the Norm2 *r2 of w.
 template <class VT>
 __global__ void __launch_bounds__(kThreads) k_lz_update(int n, const double *__restrict__ y, const VT *__restrict__ v,
-                                                       const VT *__restrict__ vprev, double *D, double *hD, const double *O,
-                                                       int b, double *__restrict__ w, const double *pp, int pcount, RedSlot out,
-                                                       Norm2 *r2) {
+                                                       const VT *__restrict__ vprev, const double *D, const double *O, int b,
+                                                       double *__restrict__ w, RedSlot out, Norm2 *r2) {
   pdl_wait();
-  // The first element's operands are loaded before the partial sums, so that both L2 round
-  // trips overlap (at solver sizes one element is often all a thread has).
-  const int i0 = blockIdx.x * kThreads + threadIdx.x, stride = gridDim.x * kThreads;
-  double y0 = 0.0, v0 = 0.0, p0 = 0.0;
-  if (i0 < n) {
-    y0 = y[i0];
-    v0 = (double)v[i0];
-    if (b > 0) p0 = (double)vprev[i0];
-  }
-  double d;
-  if (pcount > 0) {
-    d = sum_partials(pp, pcount);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      D[b] = d;
-      hD[b] = d;
-    }
-  } else {
-    d = D[b];
-  }
-  const double o = (b > 0) ? O[b] : 0.0;
+  const double d = D[b], o = (b > 0) ? O[b] : 0.0;
   double acc = 0.0;
-  auto step = [&](int i, double yi, double vi, double pi) {
-    double wi = yi - d * vi;
-    if (b > 0) wi = wi - o * pi;
+  for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
+    double wi = y[i] - d * (double)v[i];
+    if (b > 0) wi = wi - o * (double)vprev[i];
     w[i] = wi;
     acc += wi * wi;
-  };
-  if (i0 < n) step(i0, y0, v0, p0);
-  for (int i = i0 + stride; i < n; i += stride) step(i, y[i], (double)v[i], b > 0 ? (double)vprev[i] : 0.0);
+  }
   pdl_trigger();
-  if (r2)
-    grid_reduce(acc, out, [&](double t) { set_norm2(r2, t); });
-  else
-    block_partial(acc, out.partials);
+  grid_reduce(acc, out, [&](double t) { set_norm2(r2, t); });
 }
 
 // c[j] = <V_j, w> for j < nvec (one block per vector; fixed order within the block).
@@ -376,12 +441,97 @@ struct EpiCgDot {
 
 // Iteration it: alpha = rrs[it&1] / <p,y> (the product's pcount partials in pp); x += a p;
 // r -= a y; block partials of <r,r> into up (:51-63).
-__global__ void k_cg_update(int n, const double *__restrict__ p, const double *__restrict__ y, double *__restrict__ x,
-                            double *__restrict__ r, const Scalars *S, int it, const double *pp, int pcount, double *up);
+template <int T>
+__global__ void __launch_bounds__(T) k_cg_update(int n, const double *__restrict__ p, const double *__restrict__ y,
+                                                double *__restrict__ x, double *__restrict__ r, const Scalars *S, int it,
+                                                const double *pp, int pcount, double *up) {
+  __shared__ double s_a;
+  pdl_wait();
+  if (*((volatile const int *)&S->done)) return;
+  // the first elements' operands in flight before the partial sums (see k_lz_step)
+  const int i0 = blockIdx.x * T + threadIdx.x, stride = gridDim.x * T;
+  constexpr int U = kStepAhead;
+  double x0[U], p0[U], r0[U], y0[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int i = i0 + u * stride;
+    const bool in = i < n;
+    x0[u] = in ? x[i] : 0.0;
+    p0[u] = in ? p[i] : 0.0;
+    r0[u] = in ? r[i] : 0.0;
+    y0[u] = in ? y[i] : 0.0;
+  }
+  double t[1] = {partials_share(pp, pcount)};
+  block_sums<T, 1>(t);
+  if (threadIdx.x == 0) s_a = S->rrs[it & 1] / t[0];   // one division per block
+  __syncthreads();
+  const double a = s_a;
+  double acc = 0.0;
+  auto step = [&](int i, double xi, double pi, double ri, double yi) {
+    x[i] = xi + a * pi;
+    const double rn = ri - a * yi;
+    r[i] = rn;
+    acc += rn * rn;
+  };
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (i0 + u * stride < n) step(i0 + u * stride, x0[u], p0[u], r0[u], y0[u]);
+#pragma unroll 2
+  for (int i = i0 + U * stride; i < n; i += stride) step(i, x[i], p[i], r[i], y[i]);
+  pdl_trigger();
+  double u1[1] = {acc};
+  block_sums<T, 1>(u1);
+  if (threadIdx.x == 0) up[blockIdx.x] = u1[0];
+}
+
 // Iteration it: <r,r> from the update's ucount partials; convergence (<r,r> < acc_thr) or the
 // iteration limit ends the solve (block 0 records it); otherwise p = r + beta p (:64-95).
-__global__ void k_cg_direction(int n, const double *__restrict__ r, double *__restrict__ p, Scalars *S, int it, int max_step,
-                               double acc_thr, const double *up, int ucount, Progress *prog);
+template <int T>
+__global__ void __launch_bounds__(T) k_cg_direction(int n, const double *__restrict__ r, double *__restrict__ p, Scalars *S, int it,
+                                                   int max_step, double acc_thr, const double *up, int ucount, Progress *prog) {
+  __shared__ double s_b;
+  __shared__ int s_stop;
+  pdl_wait();
+  if (*((volatile const int *)&S->done)) return;
+  const int i0 = blockIdx.x * T + threadIdx.x, stride = gridDim.x * T;
+  constexpr int U = kStepAhead;
+  double r0[U], p0[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int i = i0 + u * stride;
+    const bool in = i < n;
+    r0[u] = in ? r[i] : 0.0;
+    p0[u] = in ? p[i] : 0.0;
+  }
+  double t[1] = {partials_share(up, ucount)};
+  block_sums<T, 1>(t);
+  if (threadIdx.x == 0) {
+    const bool converged = t[0] < acc_thr, last = it >= max_step - 1;
+    if (blockIdx.x == 0) {
+      if (converged) {
+        S->done = 1;
+        S->iters = it;
+      } else if (last) {
+        S->done = 2;
+        S->iters = max_step;
+      }
+      S->rrs[(it + 1) & 1] = t[0];   // the other slot: this kernel's blocks read rrs[it & 1]
+      prog->done = S->done;
+      prog->stamp = it;
+    }
+    s_stop = converged || last;   // the same decision in every block
+    s_b = t[0] / S->rrs[it & 1];
+  }
+  __syncthreads();
+  if (s_stop) return;
+  const double b = s_b;
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (i0 + u * stride < n) p[i0 + u * stride] = r0[u] + b * p0[u];
+#pragma unroll 2
+  for (int i = i0 + U * stride; i < n; i += stride) p[i] = r[i] + b * p[i];
+  pdl_trigger();
+}
 
 // ---- MINRES (sml/MINIMUM_RESIDUAL_SYM.c) ----------------------------------------------
 
@@ -434,6 +584,7 @@ __global__ void k_mr_update(int n, const double *__restrict__ v1n, const double 
 //   template <class XT, class Epi> void apply(const XT *x, Scale sc,
 //        double sigma, const int *gate, const Epi &epi, RedSlot slot, cudaStream_t st) const;
 //   int grid() const;   // apply grid (workspace sizing; number of block partials a product leaves)
+//   int grid32() const; // the same of the FP32 product
 //   long nnz() const;   // stored elements (or an estimate; 0 if unknown)
 // ---------------------------------------------------------------------------------
 
@@ -511,31 +662,25 @@ struct KrylovBasis {
   T *vec(int j) const { return V + (size_t)j * n; }
 };
 
-// Stored elements a product block needs before the FP64 Lanczos (LzSteps64) leaves its
-// reductions to the consumer.  DG_DEFER_REDUCTIONS=0 / =1 forces the last-block / consumer form
-// (in the FP64 form both give bitwise the same values); unset, the work per block decides.
-constexpr long kLzDeferWork = 6144;
+// The mixed form (LzStepsMixed) leaves its reductions to the consumer: its partials are FP32 pairs
+// that every consumer block merges on the FP32 pipes, which costs less than the serial tail of the
+// last-block form.  DG_DEFER_REDUCTIONS=0 forces the last-block form.
 inline int defer_override() {
   const char *e = std::getenv("DG_DEFER_REDUCTIONS");
   if (e && e[0] && !e[1] && (e[0] == '0' || e[0] == '1')) return e[0] == '1';
   return -1;
 }
-inline bool lz_defer(long nnz, int grid) {
-  const int o = defer_override();
-  return o >= 0 ? o == 1 : nnz >= kLzDeferWork * (long)grid;
-}
-// The mixed form (LzStepsMixed) leaves them to the consumer at every size unless forced: its
-// partials are FP32 pairs that every consumer block merges on the FP32 pipes, which costs less
-// than the serial tail of the last-block form (FP64 partials would cost each consumer block
-// FP64 adds, hence the work threshold above).
 inline bool lz_defer_mixed() {
   const int o = defer_override();
   return o >= 0 ? o == 1 : true;
 }
 
-// FP64 form (the reference's LANCZOS*): the product normalises w on the fly and stores v_b
-// into the basis; the update kernel forms w_{b+1} by the three-term recurrence, plus two
-// Gram-Schmidt passes when cfg.reorth (dense path).
+// FP64 form (the reference's LANCZOS*): two kernels a step, the product of the unnormalised w and
+// k_lz_step, which normalises it, stores v_b into the basis and forms w_{b+1} by the three-term
+// recurrence.  Neither has a last-block reduction; the product waits for no scalar.  (With the
+// product scaling its input, every one of its blocks first summed the partials of <w,w> and formed
+// a square root and a division: 10 us of a 127 us product of the Hubbard m=512 superblock.)  The dense
+// path (cfg.reorth) adds two Gram-Schmidt passes and keeps the scaling product.
 template <class Opl>
 struct LzSteps64 {
   const Opl &op;
@@ -545,46 +690,39 @@ struct LzSteps64 {
   double *w;             // start vector in, next unnormalised Krylov vector
   DevBuf<double> y, c;
   KrylovBasis<double> B;
-  // Reductions are left to the consuming kernel (the update sums the product's partials of
-  // <y,v>, the next product those of <w,w>) only when the product has >= kDeferWork stored
-  // elements a block: every consumer block then sums the partials itself, and each product
-  // block also forms 1/sqrt(<w,w>), ~70 FP64 warp instructions a block.  That is a latency win
-  // for a superblock product (KLM m=128: 8 k elements a block) but a throughput loss for an ED
-  // product of short rows (XXZ L=22: 3.5 k), where the producers' last blocks do it once.
-  bool defer;
   LzSteps64(const Opl &o, const LanczosCfg &cf, Workspace &w_, LzState &z_, double *w_dev)
-      : op(o), cfg(cf), ws(w_), z(z_), w(w_dev), y(z_.n), c(z_.cap_max + 1), B(z_.n, w_.st),
-        defer(lz_defer(o.nnz(), o.grid())) {}
-  void begin_cycle() {}
+      : op(o), cfg(cf), ws(w_), z(z_), w(w_dev), y(z_.n), c(z_.cap_max + 1), B(z_.n, w_.st) {}
+  void begin_cycle() {
+    if (cfg.reorth) return;
+    k_scale_rsqrt<double><<<ws.vgrid, kThreads, 0, ws.st>>>(w, z.n, &ws.S()->r2); ::dg::count_launch();
+    DG_CUDA(cudaGetLastError());
+  }
   void step(int b) {
     cudaStream_t st = ws.st;
     const int n = z.n;
     Scalars *S = ws.S();
     const RedSlot slot = ws.slot();
     B.ensure(b + 1, z.cap_max);
-    // 1/||w||: from the Norm2 of the start / restart vector, of a reorthogonalisation pass or
-    // of the previous update's last block; or, when the product has work enough per block to
-    // absorb it, summed by every product block from the previous update's block partials.
-    const Scale sc = (b > 0 && !cfg.reorth && defer) ? Scale::partials(ws.partials2.get(), ws.vgrid) : Scale::norm2(&S->r2);
-    if (defer) {
-      EpiLanczos<double, double, true> epi{y.get(), B.vec(b), z.D.get(), z.O.get(), z.hD.d, z.hO.d, b};
-      op.apply(w, sc, 0.0, (const int *)nullptr, epi, slot, st);
-    } else {
-      EpiLanczos<double, double, false> epi{y.get(), B.vec(b), z.D.get(), z.O.get(), z.hD.d, z.hO.d, b};
-      op.apply(w, sc, 0.0, (const int *)nullptr, epi, slot, st);
-    }
-    ++z.spmv;
     const double *vprev = (b > 0) ? B.vec(b - 1) : nullptr;
-    launch_pdl(k_lz_update<double>, ws.vgrid, kThreads, st, n, (const double *)y.get(), (const double *)B.vec(b), vprev,
-               z.D.get(), z.hD.d, (const double *)z.O.get(), b, w, (const double *)slot.partials, defer ? op.grid() : 0,
-               RedSlot{ws.partials2.get(), ws.ticket.get()}, defer ? (Norm2 *)nullptr : &S->r2);
-    if (cfg.reorth) {
-      for (int pass = 0; pass < 2; ++pass) {
-        k_multidot<double><<<std::min(b + 1, 1024), kThreads, 0, st>>>(B.V, n, b + 1, w, n, c.get()); ::dg::count_launch();
-        k_multisub<double><<<ws.vgrid, kThreads, 0, st>>>(B.V, n, b + 1, c.get(), w, n, &S->r2, slot); ::dg::count_launch();
-      }
-      DG_CUDA(cudaGetLastError());
+    ++z.spmv;
+    if (!cfg.reorth) {
+      op.apply(w, Scale{}, 0.0, (const int *)nullptr, EpiLzRaw{y.get()}, slot, st);
+      // <w,w> partials alternate: a step reads the last one's while it writes its own
+      double *const rp[2] = {ws.partials2.get(), ws.partials3.get()};
+      launch_pdl(ws.uthreads == kThreads ? k_lz_step<kThreads> : k_lz_step<512>, ws.ugrid, ws.uthreads, st, n, (const double *)y.get(),
+                 w, B.vec(b), vprev, z.D.get(), z.O.get(), z.hD.d, z.hO.d, b, (const double *)slot.partials, op.grid(),
+                 (const double *)rp[(b + 1) & 1], ws.ugrid, rp[b & 1]);
+      return;
     }
+    EpiLanczos<double, double, false> epi{y.get(), B.vec(b), z.D.get(), z.O.get(), z.hD.d, z.hO.d, b};
+    op.apply(w, Scale::norm2(&S->r2), 0.0, (const int *)nullptr, epi, slot, st);
+    launch_pdl(k_lz_update<double>, ws.vgrid, kThreads, st, n, (const double *)y.get(), (const double *)B.vec(b), vprev,
+               (const double *)z.D.get(), (const double *)z.O.get(), b, w, RedSlot{ws.partials2.get(), ws.ticket.get()}, &S->r2);
+    for (int pass = 0; pass < 2; ++pass) {
+      k_multidot<double><<<std::min(b + 1, 1024), kThreads, 0, st>>>(B.V, n, b + 1, w, n, c.get()); ::dg::count_launch();
+      k_multisub<double><<<ws.vgrid, kThreads, 0, st>>>(B.V, n, b + 1, c.get(), w, n, &S->r2, slot); ::dg::count_launch();
+    }
+    DG_CUDA(cudaGetLastError());
   }
   // dst = sum_{j<k} s_j v_j with <dst,dst> in S->r2
   void combine(int k, const std::vector<double> &s, double *dst) {
@@ -640,7 +778,7 @@ struct LzStepsMixed {
     Norm2 *r2 = defer ? (Norm2 *)nullptr : &S->r2;
     if (!cfg.mixed_reorth) {
       launch_pdl(k_mx_update, ws.vgrid, kThreads, st, B.V, (long)n, b, (const double *)sig.get(), (const float *)y.get(),
-                 z.D.get(), z.hD.d, (const double *)z.O.get(), n, (const double *)slot.partials, defer ? op.grid() : 0, r2slot,
+                 z.D.get(), z.hD.d, (const double *)z.O.get(), n, (const double *)slot.partials, defer ? op.grid32() : 0, r2slot,
                  r2);
       return;
     }
@@ -652,7 +790,7 @@ struct LzStepsMixed {
     // the three-term residual the ratio is about 1 and orthogonality stays at the FP32 level.
     const RedSlot scratch{ws.partials3.get(), ws.ticket.get()};
     launch_pdl(k_mx_update, ws.vgrid, kThreads, st, B.V, (long)n, b, (const double *)sig.get(), (const float *)y.get(), z.D.get(),
-               z.hD.d, (const double *)z.O.get(), n, (const double *)slot.partials, defer ? op.grid() : 0, scratch,
+               z.hD.d, (const double *)z.O.get(), n, (const double *)slot.partials, defer ? op.grid32() : 0, scratch,
                (Norm2 *)nullptr);
     const int nvec = b + 1;
     const float *w3 = B.vec(b + 1);
@@ -851,10 +989,11 @@ IterResult cg_core(const Opl &op, double sigma, const double *b_dev, double *x_d
   auto enqueue_to = [&](int last) {
     for (int it = enq + 1; it <= last; ++it) {
       op.apply(p.get(), Scale{}, sigma, &S->done, EpiCgDot{y.get()}, slot, st);
-      launch_pdl(k_cg_update, ws.vgrid, kThreads, st, n, (const double *)p.get(), (const double *)y.get(), x_dev, r.get(),
-                 (const Scalars *)S, it, (const double *)slot.partials, pgrid, up);
-      launch_pdl(k_cg_direction, ws.vgrid, kThreads, st, n, (const double *)r.get(), p.get(), S, it, max_step, acc,
-                 (const double *)up, ws.vgrid, ws.prog.d);
+      launch_pdl(ws.uthreads == kThreads ? k_cg_update<kThreads> : k_cg_update<512>, ws.ugrid, ws.uthreads, st, n,
+                 (const double *)p.get(), (const double *)y.get(), x_dev, r.get(), (const Scalars *)S, it,
+                 (const double *)slot.partials, pgrid, up);
+      launch_pdl(ws.uthreads == kThreads ? k_cg_direction<kThreads> : k_cg_direction<512>, ws.ugrid, ws.uthreads, st, n,
+                 (const double *)r.get(), p.get(), S, it, max_step, acc, (const double *)up, ws.ugrid, ws.prog.d);
     }
     DG_CUDA(cudaGetLastError());
     enq = std::max(enq, last);

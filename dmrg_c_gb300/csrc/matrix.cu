@@ -397,6 +397,15 @@ void launch_validate(const int64_t *row, const int *col, int n, long nnz, int lo
   k_validate<<<warp_grid(n), kThreads, 0, st>>>(row, col, n, nnz, lower, bad); ::dg::count_launch();
 }
 
+// Blocks a SM of the sliced-ELL grids: of the FP64 product's pipelined form, and of the others.
+constexpr int kSellBpsPipe = 3, kSellBps = 16;
+
+static int sell_grid_for(const dg_matrix *m, int ws, int bps) {
+  const int groups = kWarps / ws;
+  const long need = (m->nslices + groups - 1) / groups;
+  return (int)std::max(1L, std::min(need, (long)sm_count() * bps));
+}
+
 void build_sell(dg_matrix *m, cudaStream_t st, int window) {
   const int n = m->n;
   const int nwin = (n + kSellWindow - 1) / kSellWindow;
@@ -477,14 +486,12 @@ void build_sell(dg_matrix *m, cudaStream_t st, int window) {
     if (sell_uses_deltas(m->sell_variant32)) m->sell_variant32 = V_U8;
   }
   DG_CUDA(cudaGetLastError());
-  choose_sell_shape(nslices, total, &m->sell_ws, &m->sell_grid);
-  // Measured on GB300.  Superblocks (3.6 k - 228 k rows, 24+ stored elements a row): with one
-  // or two warps per slice the software-pipelined 8-element groups are fastest, with four or
-  // eight the 16-element groups (more loads in flight per warp).  ED Hamiltonians (0.7 - 0.85 M
-  // rows of ~12 elements, one warp per slice): a whole row fits one 16-element group, and the
-  // pipelined form, which has no second group to overlap, is the slowest (12-14 % behind).
-  const double per_row = (double)total / ((double)nslices * kSellC);
-  m->sell_variant = (m->sell_ws >= 4 || per_row < 24.0) ? V_U16 : V_PIPE8;
+  const SellShape f64 = choose_sell_shape(n, nslices, total, false), f32 = choose_sell_shape(n, nslices, total, true);
+  m->sell_ws = f64.ws;
+  m->sell_variant = f64.variant;
+  m->sell_grid = f64.grid;
+  m->sell_ws32 = f32.ws;
+  m->sell_grid32 = f32.grid;
   // The FP32 product on the delta stream (6 bytes an element instead of 8): on the Hubbard m=512
   // superblock of a DMRG sweep (238 k rows of 236 stored elements) 8-element groups with the next chunk prefetched into L2 took
   // 79 us at one warp per slice and 81 at two, against 92 us for the 32-bit columns.  One warp a
@@ -492,32 +499,47 @@ void build_sell(dg_matrix *m, cudaStream_t st, int window) {
   // gains nothing from the deltas and keeps its variant.
   if (m->has_d16()) {
     m->sell_variant32 = V_D8;
-    m->sell_ws32 = (m->sell_ws <= 2 && (long)nslices >= 24L * sm_count()) ? 1 : m->sell_ws;
-  } else {
-    if (sell_uses_deltas(m->sell_variant32)) m->sell_variant32 = V_U8;
-    m->sell_ws32 = m->sell_ws;
+    if (m->sell_ws32 <= 2 && (long)nslices >= 24L * sm_count()) {
+      m->sell_ws32 = 1;
+      m->sell_grid32 = sell_grid_for(m, 1, kSellBps);
+    }
+  } else if (sell_uses_deltas(m->sell_variant32)) {
+    m->sell_variant32 = V_U8;
   }
   DG_CUDA(cudaStreamSynchronize(st));
   m->sell_checkpoints = (long)nchk;
 }
 
-void choose_sell_shape(int nslices, long stored, int *ws, int *grid) {
+SellShape choose_sell_shape(long n, int nslices, long stored, bool f32) {
   const long target_warps = (long)sm_count() * 96;
-  const double per_row = nslices > 0 ? (double)stored / ((double)nslices * kSellC) : 0.0;
+  // Elements a row: over the rows there are for the FP64 product; the FP32 product keeps its slots
+  // (its sums are split over the warps it always had).
+  const double per_row = f32 ? (nslices > 0 ? (double)stored / ((double)nslices * kSellC) : 0.0) : (double)stored / std::max(1L, n);
   int w = 1;
   if (per_row >= 24.0) {
     // Split a slice over more warps while each keeps >= 32 elements of every row, or, for
-    // matrices too small to fill the GPU, while each keeps >= 8 and the doubled warp count
-    // stays under a quarter of the target.
+    // matrices too small to fill the GPU, while each keeps >= 8 and all of them run at once.
+    // Measured (FP64, L2 warm, us a product at 2 / 4 / 8 warps): XXZ m=64 (128 slices of 66) - / 11.5 /
+    // 10.0, Kondo m=127 (1,600 of 59) 18.2 / 16.9 / -, Hubbard m=200 (1,280 of 103) 20.8 / 18.9 / 20.1.
+    const long together = f32 ? target_warps / 4 : (long)sm_count() * 48;
     w = 2;
     while (w < 8 && (long)nslices * w < target_warps &&
-           (per_row / (2 * w) >= 32.0 || ((long)nslices * 2 * w <= target_warps / 4 && per_row / (2 * w) >= 8.0)))
+           (per_row / (2 * w) >= 32.0 || ((long)nslices * 2 * w <= together && per_row / (2 * w) >= 8.0)))
       w <<= 1;
   }
+  // Variant of the FP64 product.  Superblocks: the software-pipelined 8-element groups, except where
+  // four or eight warps a slice have >= 32 elements each (16-element groups: Hubbard m=300 41.4 against
+  // 46.0 us).  ED Hamiltonians (0.7 - 0.85 M rows of ~12 elements, one warp per slice): a whole row
+  // fits one 16-element group, and the pipelined form, which has no second group to overlap, is the
+  // slowest (12-14 % behind).
+  const int var = per_row < 24.0 || (w >= 4 && per_row / w >= 32.0) ? V_U16 : V_PIPE8;
   const int groups = kWarps / w;
   const long need = (nslices + groups - 1) / groups;
-  *ws = w;
-  *grid = (int)std::max(1L, std::min(need, (long)sm_count() * 16));
+  // The pipelined form runs three blocks a SM (78 registers): one wave of blocks that walk the slices
+  // beats several (Hubbard m=512 126 against 130 us, Kondo m=127 16.9 against 17.4) and leaves a
+  // quarter of the reduction partials for the next kernel to sum.
+  const int bps = !f32 && var == V_PIPE8 ? kSellBpsPipe : kSellBps;
+  return SellShape{w, var, (int)std::max(1L, std::min(need, (long)sm_count() * bps))};
 }
 
 dg_matrix *matrix_from_device(int n, long nnz_in, const long *row_d, const int *col_d, const double *val_d, int storage,
@@ -682,6 +704,7 @@ int dg_matrix_set_sell_shape(dg_matrix *m, int warps_per_slice, int grid) {
     m->sell_ws = warps_per_slice;
     m->sell_ws32 = warps_per_slice;
     m->sell_grid = grid;
+    m->sell_grid32 = grid;
     m->format = DG_FORMAT_SELL;
   });
 }
@@ -750,7 +773,7 @@ int dg_spmv_f32(dg_matrix *m, const float *x, float *y) {
       yp = yb.get();
     }
     if (m->format == DG_FORMAT_SELL)
-      launch_sell(m->sell32(), m->sell_grid, xp, Scale{}, 0.0, (const int *)nullptr,
+      launch_sell(m->sell32(), m->sell_grid32, xp, Scale{}, 0.0, (const int *)nullptr,
                   EpiStore<float>{yp}, RedSlot{nullptr, nullptr}, st);
     else
       launch_apply(m->op32(), m->lanes, m->grid, m->n, xp, Scale{}, 0.0, (const int *)nullptr,
@@ -814,7 +837,7 @@ void profile_apply(dg_matrix *m, const XT *x_dev, double *y_dev, int iters, size
   DG_REQUIRE(m && x_dev && y_dev && ms_per_launch && iters > 0, DG_ERR_ARG, "bad argument");
   DG_REQUIRE(is_device_ptr(x_dev) && is_device_ptr(y_dev), DG_ERR_ARG, "profiling needs device vectors");
   cudaStream_t st = stream();
-  DevBuf<double> partials(std::max(m->grid, m->sell_grid)), out(1);
+  DevBuf<double> partials(std::max(m->grid, std::max(m->sell_grid, m->sell_grid32))), out(1);
   DevBuf<unsigned> ticket(1);
   DG_CUDA(cudaMemsetAsync(ticket.get(), 0, sizeof(unsigned), st));
   flush_bytes = (flush_bytes + 15) / 16 * 16;
@@ -885,12 +908,6 @@ ShapeClass shape_class(const dg_matrix *m) {
   return ShapeClass{logn, (int)std::min(per, 1L << 20), m->has32 ? 1 : 0};
 }
 
-int sell_grid_for(const dg_matrix *m, int ws, int bps) {
-  const int groups = kWarps / ws;
-  const long need = (m->nslices + groups - 1) / groups;
-  return (int)std::max(1L, std::min(need, (long)sm_count() * bps));
-}
-
 // A variant this matrix can run: the delta variants fall back to the same kernel on 32-bit
 // columns when a matrix of the class has no delta stream.
 int runnable_variant(const dg_matrix *m, int v) {
@@ -902,7 +919,7 @@ void apply_shape(dg_matrix *m, const TunedShape &t) {
   m->format = DG_FORMAT_SELL;
   m->sell_ws = t.ws;
   m->sell_variant = runnable_variant(m, t.variant);
-  m->sell_grid = sell_grid_for(m, t.ws, t.bps);
+  m->sell_grid = m->sell_grid32 = sell_grid_for(m, t.ws, t.bps);
   m->sell_ws32 = t.ws32;
   m->sell_variant32 = runnable_variant(m, t.variant32);
 }
@@ -943,10 +960,10 @@ TunedShape tune_sell(dg_matrix *m, int iters) {
   auto candidate = [&](int ws, int v) {   // the streamed variants run one warp a slice
     return (!sell_uses_deltas(v) || m->has_d16()) && !((v == V_TMA || v == V_TMA16) && ws > 1);
   };
-  // the build heuristic's shape first: its grid is one of the two candidates' (16 blocks a SM)
+  // the build heuristic's shape first
   m->format = DG_FORMAT_SELL;
-  TunedShape best{m->sell_ws, m->sell_variant, m->sell_ws32, m->sell_variant32, 16};
-  m->sell_grid = sell_grid_for(m, best.ws, best.bps);
+  TunedShape best{m->sell_ws, m->sell_variant, m->sell_ws32, m->sell_variant32, m->sell_variant == V_PIPE8 ? kSellBpsPipe : kSellBps};
+  m->sell_grid = m->sell_grid32 = sell_grid_for(m, best.ws, best.bps);
   float best_ms = time_it(false);
   for (int ws = 1; ws <= 8; ws <<= 1)
     for (int v = 0; v < V_COUNT; ++v) {
@@ -1114,7 +1131,7 @@ int dg_matrix_autotune(dg_matrix *m, int iters, dg_tune_result *out) {
             m->format = DG_FORMAT_SELL;
             m->sell_ws = ws;
             m->sell_variant = var;
-            m->sell_grid = grid;
+            m->sell_grid = m->sell_grid32 = grid;
             const float ms = time_it();
             ++tried;
             if (ms < best.ms) best = dg_tune_result{DG_FORMAT_SELL, ws, var, grid, ms, 0, windows[wi]};
@@ -1142,7 +1159,7 @@ int dg_matrix_autotune(dg_matrix *m, int iters, dg_tune_result *out) {
       m->sell_ws = best.shape;
       m->sell_ws32 = best.shape;
       m->sell_variant = best.variant;
-      m->sell_grid = best.grid;
+      m->sell_grid = m->sell_grid32 = best.grid;
       if (sell_uses_deltas(m->sell_variant32) && !m->has_d16()) m->sell_variant32 = V_U8;
     } else {
       m->format = DG_FORMAT_CSR;

@@ -23,8 +23,9 @@ struct dg_matrix {
   int nslices = 0;
   long nnz_sell = 0;               // stored elements including padding
   int sell_grid = 1;
+  int sell_grid32 = 1;             // grid of the FP32 (mixed) product
   int sell_ws = 1;                 // warps per slice
-  int sell_ws32 = 1;               // warps per slice of the FP32 (mixed) product (same grid)
+  int sell_ws32 = 1;               // warps per slice of the FP32 (mixed) product
   int sell_variant = 1;            // SellVariant of the FP64 product (V_U8)
   int sell_variant32 = 1;          // SellVariant of the FP32 (mixed) product: 8-element groups
                                    // measured fastest there at every warps-per-slice count
@@ -132,10 +133,12 @@ void launch_sell(const SellOp<VT> &op, int grid, const XT *x, Scale sc, double s
   DG_CUDA(cudaGetLastError());
 }
 
-// Warps per slice and grid for the sliced-ELL kernel (heuristic from measured sweeps):
-// short rows (ED matrices) one warp per slice; otherwise split slices over more warps while
-// each keeps >= 32 elements of every row (or >= 8 for matrices too small to fill the GPU).
-void choose_sell_shape(int nslices, long stored, int *ws, int *grid);
+// Warps per slice, variant and grid of the sliced-ELL kernel for n rows with `stored` elements
+// (matrix.cu; heuristic from measured sweeps).
+struct SellShape {
+  int ws, variant, grid;
+};
+SellShape choose_sell_shape(long n, int nslices, long stored, bool f32);
 
 // Apply the matrix in its selected format with FP64 values.
 template <class XT, class Epi>
@@ -152,13 +155,14 @@ template <class Epi>
 void matrix_apply32(const dg_matrix *m, const float *x, Scale sc, double sigma, const int *gate,
                     const Epi &epi, RedSlot slot, cudaStream_t st) {
   if (m->format == DG_FORMAT_SELL)
-    launch_sell(m->sell32(), m->sell_grid, x, sc, sigma, gate, epi, slot, st);
+    launch_sell(m->sell32(), m->sell_grid32, x, sc, sigma, gate, epi, slot, st);
   else
     launch_apply(m->op32(), m->lanes, m->grid, m->n, x, sc, sigma, gate, epi, slot, st);
 }
 
 // Blocks needed by the current format (for sizing reduction partials).
 inline int matrix_grid(const dg_matrix *m) { return m->format == DG_FORMAT_SELL ? m->sell_grid : m->grid; }
+inline int matrix_grid32(const dg_matrix *m) { return m->format == DG_FORMAT_SELL ? m->sell_grid32 : m->grid; }
 
 // Checks the CRS invariants of device arrays on stream st (row offsets non-decreasing within
 // [0, nnz]; columns in [0, n), or the lower-triangle layout when lower = 1).  *bad must hold

@@ -78,6 +78,7 @@ struct RawCrsLauncher {
   int n_, lanes, grid_;
   int n() const { return n_; }
   int grid() const { return grid_; }
+  int grid32() const { return grid_; }
   long nnz() const { return 0; }
   template <class XT, class Epi>
   void apply(const XT *x, Scale sc, double sigma, const int *gate, const Epi &epi, RedSlot slot,
@@ -154,8 +155,8 @@ extern "C" int dg_cg_noalloc(int n, const long *row_dev, const int *col_dev, con
       const int last = std::min(it + chunk - 1, max_step - 1);
       for (; it <= last; ++it) {
         op.apply(p, Scale{}, sigma, &S->done, EpiCgDot{y}, slot, st);
-        k_cg_update<<<vgrid, kThreads, 0, st>>>(n, p, y, x_dev, r, S, it, partials, op.grid_, partials2); ::dg::count_launch();
-        k_cg_direction<<<vgrid, kThreads, 0, st>>>(n, r, p, S, it, max_step, acc, partials2, vgrid, prog); ::dg::count_launch();
+        k_cg_update<kThreads><<<vgrid, kThreads, 0, st>>>(n, p, y, x_dev, r, S, it, partials, op.grid_, partials2); ::dg::count_launch();
+        k_cg_direction<kThreads><<<vgrid, kThreads, 0, st>>>(n, r, p, S, it, max_step, acc, partials2, vgrid, prog); ::dg::count_launch();
       }
       DG_CUDA(cudaGetLastError());
       DG_CUDA(cudaMemcpyAsync(&done, &S->done, sizeof(int), cudaMemcpyDeviceToHost, st));

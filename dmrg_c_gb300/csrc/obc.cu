@@ -122,6 +122,7 @@ struct ObcLauncher {
   const ObcData *D;
   int n() const { return D->n; }
   int grid() const { return D->grid; }
+  int grid32() const { return D->grid; }
   long nnz() const { return (long)D->n * D->nnz_est; }   // nnz_est: elements a row
   template <class XT, class Epi>
   void apply(const XT *x, Scale sc, double sigma, const int *gate, const Epi &epi, RedSlot slot,

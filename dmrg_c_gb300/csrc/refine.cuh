@@ -153,7 +153,7 @@ RefineResult refine_core(const Opl &op, double acc, int max_outer, int max_inner
     // Pair partials: the product's <p32,q32> in slot.partials, the update's <res32,res32> in
     // partials2, the direction's <g32,p32> in partials3; each summed by every block of its consumer.
     float2 *up = reinterpret_cast<float2 *>(ws.partials2.get()), *gpp = reinterpret_cast<float2 *>(ws.partials3.get());
-    const int pgrid = op.grid();
+    const int pgrid = op.grid32();
     k_refine32_direction<<<vg, kThreads, 0, st>>>(n, res32.get(), p32.get(), g32.get(), S, 0, max_inner, (const float2 *)up, 0,
                                                   gpp, ws.prog.d); ::dg::count_launch();
     const int chunk = 8;

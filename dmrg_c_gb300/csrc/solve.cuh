@@ -26,6 +26,7 @@ struct CrsLauncher {
   const dg_matrix *m;
   int n() const { return m->n; }
   int grid() const { return matrix_grid(m); }
+  int grid32() const { return matrix_grid32(m); }
   long nnz() const { return m->nnz; }
   template <class XT, class Epi>
   void apply(const XT *x, Scale sc, double sigma, const int *gate, const Epi &epi, RedSlot slot,
@@ -111,7 +112,7 @@ SolveOut solve_ground_state(const Opl &op, const dg_solver_params &p, const doub
   DG_REQUIRE(p.lanczos_max_step > p.lanczos_min_step || dense_route(p, n), DG_ERR_ARG, "max_step=%d must exceed min_step=%d", p.lanczos_max_step,
              p.lanczos_min_step);
   cudaStream_t st = stream();
-  Workspace ws(n, op.grid(), st);
+  Workspace ws(n, std::max(op.grid(), op.grid32()), st);
   VecArg out(eigvec, n, false, true, st);
   DevBuf<double> w(n);
   if (guess) {
@@ -192,7 +193,7 @@ template <class Opl>
 SolveOut solve_inverse_iteration(const Opl &op, const dg_solver_params &p, double eig_val, double *eigvec, bool shifted_check) {
   const int n = op.n();
   cudaStream_t st = stream();
-  Workspace ws(n, op.grid(), st);
+  Workspace ws(n, std::max(op.grid(), op.grid32()), st);
   VecArg v(eigvec, n, true, true, st);
   SolveOut o;
   int sp = 0;
@@ -211,7 +212,7 @@ template <class Opl>
 IterResult solve_linear(const Opl &op, double sigma, const double *b, double *x, double acc, int max_step, bool minres) {
   const int n = op.n();
   cudaStream_t st = stream();
-  Workspace ws(n, op.grid(), st);
+  Workspace ws(n, std::max(op.grid(), op.grid32()), st);
   VecArg bv(b, n, true, false, st);
   VecArg xv(x, n, true, true, st);
   int sp = 0;
@@ -224,7 +225,7 @@ IterResult solve_linear(const Opl &op, double sigma, const double *b, double *x,
 template <class Opl>
 double solve_residual(const Opl &op, const double *x, double sigma, double lambda) {
   cudaStream_t st = stream();
-  Workspace ws(op.n(), op.grid(), st);
+  Workspace ws(op.n(), std::max(op.grid(), op.grid32()), st);
   VecArg xv(x, op.n(), true, false, st);
   return residual_core(op, xv.dev, sigma, lambda, ws);
 }
