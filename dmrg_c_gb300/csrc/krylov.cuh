@@ -28,6 +28,7 @@
 #include "apply.cuh"
 #include "sell.cuh"
 #include "common.cuh"
+#include "dense.cuh"
 #include "tridiag.h"
 
 namespace dg {
@@ -585,6 +586,7 @@ __global__ void k_mr_update(int n, const double *__restrict__ v1n, const double 
 //        double sigma, const int *gate, const Epi &epi, RedSlot slot, cudaStream_t st) const;
 //   int grid() const;   // apply grid (workspace sizing; number of block partials a product leaves)
 //   int grid32() const; // the same of the FP32 product
+//   const dg_matrix *matrix() const;   // the CRS behind the operator, null if there is none
 //   long nnz() const;   // stored elements (or an estimate; 0 if unknown)
 // ---------------------------------------------------------------------------------
 
@@ -680,7 +682,8 @@ inline bool lz_defer_mixed() {
 // recurrence.  Neither has a last-block reduction; the product waits for no scalar.  (With the
 // product scaling its input, every one of its blocks first summed the partials of <w,w> and formed
 // a square root and a division: 10 us of a 127 us product of the Hubbard m=512 superblock.)  The dense
-// path (cfg.reorth) adds two Gram-Schmidt passes and keeps the scaling product.
+// path (cfg.reorth) adds two Gram-Schmidt passes: one cluster kernel a step (dense.cuh) up to 1,024
+// states, else the scaling product, the recurrence and the passes as kernels of their own.
 template <class Opl>
 struct LzSteps64 {
   const Opl &op;
@@ -714,6 +717,9 @@ struct LzSteps64 {
                  (const double *)rp[(b + 1) & 1], ws.ugrid, rp[b & 1]);
       return;
     }
+    if (op.matrix() && launch_dense_step(op.matrix(), DenseStep{n, b, nullptr, nullptr, nullptr, B.V, w, z.D.get(), z.O.get(), z.hD.d,
+                                                                z.hO.d, &S->r2}, st))
+      return;
     EpiLanczos<double, double, false> epi{y.get(), B.vec(b), z.D.get(), z.O.get(), z.hD.d, z.hO.d, b};
     op.apply(w, Scale::norm2(&S->r2), 0.0, (const int *)nullptr, epi, slot, st);
     launch_pdl(k_lz_update<double>, ws.vgrid, kThreads, st, n, (const double *)y.get(), (const double *)B.vec(b), vprev,
