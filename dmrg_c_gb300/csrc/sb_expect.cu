@@ -167,13 +167,13 @@ __global__ void __launch_bounds__(kThreads) k_sb_expect_sum(const double *__rest
 struct PairView {
   int R, B, dim_RR, d;
   const int *run_ll, *run_lr, *run_blk, *blk_run0, *blk_Q, *pair_run, *rrrl_pos;
-  const int64_t *blk_base, *rho_off, *sig_off, *q_off, *rho_tri, *sig_tri;
+  const int64_t *blk_base, *rho_off, *sig_off, *q_off, *rho_tri;
 };
 
 PairView pair_view(const SbPairs &P) {
   return PairView{P.R, P.B, P.dim_RR, P.d, P.d_run_ll.get(), P.d_run_lr.get(), P.d_run_blk.get(), P.d_blk_run0.get(), P.d_blk_Q.get(),
                   P.d_pair_run.get(), P.d_rrrl_pos.get(), P.d_blk_base.get(), P.d_rho_off.get(), P.d_sig_off.get(), P.d_q_off.get(),
-                  P.d_rho_tri.get(), P.d_sig_tri.get()};
+                  P.d_rho_tri.get()};
 }
 
 // Largest g in [0, B) with off[g] <= e (off ascending, off[0] = 0).
@@ -202,69 +202,120 @@ __device__ __forceinline__ void tri_index(int64_t loc, int n, int &p, int &q) {
   q = r + (int)(loc - start(r));
 }
 
-// The sum of x[k*stride] * y[k*stride] over k < len, in k order: EXACT rounds every product and
-// sum as written (the reference's density-matrix entries, bitwise), else fused multiply-adds (half
-// the FP64 instructions; for the expectation values, which only need the value to 1e-16).
-template <bool EXACT>
-__device__ __forceinline__ double dot_strided(const double *__restrict__ x, const double *__restrict__ y, int len, int64_t stride) {
-  double acc = 0.0;
-  for (int k = 0; k < len; ++k) {
-    const double a = x[(int64_t)k * stride], b = y[(int64_t)k * stride];
-    acc = EXACT ? __dadd_rn(acc, __dmul_rn(a, b)) : fma(a, b, acc);
-  }
-  return acc;
-}
-
-// rho_g[p][q] = sum_t w[row p][t] * v[row q][t] for every block, summed over t in order (with
-// EXACT and w = v these are DMRG_GET_DENSITY_MATRIX's entries, bit for bit).  SYM (w = v): only the
-// upper triangles are enumerated (every thread has an entry) and mirrored -- the products of
-// (q, p) are those of (p, q), so the mirror is the value its own sum would give.
-template <bool SYM, bool EXACT>
-__global__ void __launch_bounds__(kThreads) k_gram_rows(PairView P, const double *__restrict__ w, const double *__restrict__ v,
-                                                       double *__restrict__ rho) {
-  const int64_t *off = SYM ? P.rho_tri : P.rho_off;
-  const int64_t total = off[P.B];
+// rho_g[p][q] = sum_t v[row p][t] * v[row q][t] for every block, in t order with every product and
+// sum rounded as written: DMRG_GET_DENSITY_MATRIX's entries, bit for bit.  Only the upper triangles
+// are enumerated (every thread has an entry) and mirrored -- the products of (q, p) are those of
+// (p, q), so the mirror is the value its own sum would give.
+__global__ void __launch_bounds__(kThreads) k_gram_rows(PairView P, const double *__restrict__ v, double *__restrict__ rho) {
+  const int64_t total = P.rho_tri[P.B];
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-    const int g = find_block(off, P.B, e);
+    const int g = find_block(P.rho_tri, P.B, e);
     const int Pg = P.blk_run0[g + 1] - P.blk_run0[g], Q = P.blk_Q[g];
-    const int64_t loc = e - off[g];
     int p, q;
-    if (SYM) {
-      tri_index(loc, Pg, p, q);
-    } else {
-      p = (int)(loc / Pg);
-      q = (int)(loc - (int64_t)p * Pg);
-    }
-    const double acc = dot_strided<EXACT>(w + P.blk_base[g] + (int64_t)p * Q, v + P.blk_base[g] + (int64_t)q * Q, Q, 1);
+    tri_index(e - P.rho_tri[g], Pg, p, q);
+    const double *__restrict__ x = v + P.blk_base[g] + (int64_t)p * Q;
+    const double *__restrict__ y = v + P.blk_base[g] + (int64_t)q * Q;
+    double acc = 0.0;
+    for (int t = 0; t < Q; ++t) acc = __dadd_rn(acc, __dmul_rn(x[t], y[t]));
     double *blk = rho + P.rho_off[g];
     blk[(int64_t)p * Pg + q] = acc;
-    if (SYM) blk[(int64_t)q * Pg + p] = acc;
+    blk[(int64_t)q * Pg + p] = acc;
   }
 }
 
-// sigma_g[t][u] = sum_p w[row p][t] * v[row p][u] for every block (SYM: upper triangles, mirrored).
+// The density-matrix entries expectation values read, of every block at once.  An operator on LL leaves
+// LR as it is, so the trace meets rho only between runs of the same LR, and one on LR only between runs
+// of the same LL (sigma: the same RL, RR): with d site states about one entry in d, and the FP64
+// products of the others are not needed.  kGramParts warps per run (row of rho) or column slot (row
+// of sigma) collect the entries its row needs and share them out; kGramLanes lanes sum one, four loads
+// in flight each.  need: kNeed* bits; SYM (w = v): the upper triangles, mirrored.
+// Bound by FP64 issue where the blocks are large (an SM starts one FP64 warp instruction per ~19 cycles)
+// and by how evenly the rows fall on the SMs.  Hubbard m=512 (46 blocks of up to 199 x 198), operators at
+// all four positions: 58 us; every entry of rho and sigma, a thread each in one chain of multiply-adds:
+// 53 + 70 us in two launches; the needed ones, a lane each: 112 us.  Whole expectation call with 64
+// terms, lanes / parts / warps: 8/4/4 165 us, 8/2/4 176, 8/8/8 175, 16/2/4 190, 4/4/4 176.
+constexpr int kGramLanes = 8, kGramParts = 4, kGramWarps = 4;
+enum : int { kNeedLL = 1, kNeedLR = 2, kNeedRR = 4, kNeedRL = 8 };
+
 template <bool SYM>
-__global__ void __launch_bounds__(kThreads) k_gram_cols(PairView P, const double *__restrict__ w, const double *__restrict__ v,
-                                                       double *__restrict__ sig) {
-  const int64_t *off = SYM ? P.sig_tri : P.sig_off;
-  const int64_t total = off[P.B];
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-    const int g = find_block(off, P.B, e);
-    const int Pg = P.blk_run0[g + 1] - P.blk_run0[g], Q = P.blk_Q[g];
-    const int64_t loc = e - off[g];
-    int t, u;
-    if (SYM) {
-      tri_index(loc, Q, t, u);
-    } else {
-      t = (int)(loc / Q);
-      u = (int)(loc - (int64_t)t * Q);
+__global__ void __launch_bounds__(32 * kGramWarps) k_gram_needed(PairView P, SbStates S, int need, const double *__restrict__ w,
+                                                         const double *__restrict__ v, double *__restrict__ rho,
+                                                         double *__restrict__ sig) {
+  __shared__ int s_list[kGramWarps][64];
+  const int lane = threadIdx.x & 31;
+  int *const list = s_list[threadIdx.x >> 5];
+  const int64_t n_row = need & (kNeedLL | kNeedLR) ? P.R : 0, n_col = need & (kNeedRR | kNeedRL) ? P.q_off[P.B] : 0;
+  const int64_t nw = (int64_t)gridDim.x * kGramWarps;
+  const int sub = lane % kGramLanes, slot = lane / kGramLanes;
+  for (int64_t it = (int64_t)blockIdx.x * kGramWarps + (threadIdx.x >> 5); it < (n_row + n_col) * kGramParts; it += nw) {
+    const int64_t item = it / kGramParts;
+    const int part = (int)(it - item * kGramParts);
+    const bool rows = item < n_row;
+    const int g = rows ? P.run_blk[item] : find_block(P.q_off, P.B, item - n_row);
+    const int r0 = P.blk_run0[g], Pg = P.blk_run0[g + 1] - r0, Q = P.blk_Q[g];
+    const int64_t base = P.blk_base[g];
+    const int me = rows ? (int)item - r0 : (int)(item - n_row - P.q_off[g]);   // this row of rho_g / sigma_g
+    const int dim = rows ? Pg : Q;
+    // the two coordinates of a row: (LL, LR) of a run, (RR, RL) of a column slot
+    auto coord = [&](int k) {
+      return rows ? make_int2(P.run_ll[r0 + k], P.run_lr[r0 + k])
+                  : make_int2(S.st[DG_SB_RR][base + k], S.st[DG_SB_RL][base + k]);
+    };
+    const int2 mine = coord(me);
+    // an operator on the first coordinate keeps the second, and the other way round
+    const bool by_second = need & (rows ? kNeedLL : kNeedRR), by_first = need & (rows ? kNeedLR : kNeedRL);
+    const double *const x = w + base + (rows ? (int64_t)me * Q : me), *const y = v + base;
+    const int64_t step = rows ? 1 : Q, row_of = rows ? Q : 1;   // along the sum; from one entry to the next
+    const int len = rows ? Q : Pg;
+    double *const blk = rows ? rho + P.rho_off[g] : sig + P.sig_off[g];
+    int pending = 0;
+    for (int k0 = SYM ? me & ~31 : 0; k0 < dim || pending > 0; k0 += 32) {
+      const int k = k0 + lane;
+      bool take = false;
+      if (k < dim && (!SYM || k >= me)) {
+        const int2 c = coord(k);
+        take = (by_second && c.y == mine.y) || (by_first && c.x == mine.x);
+      }
+      const unsigned bal = __ballot_sync(0xffffffffu, take);
+      if (take) list[pending + __popc(bal & ((1u << lane) - 1u))] = k;
+      pending += __popc(bal);
+      __syncwarp();
+      if (pending < 32 && k0 + 32 < dim) continue;
+      const int cnt = min(pending, 32);
+      for (int e0 = 0; e0 < cnt; e0 += 32 / kGramLanes * kGramParts) {
+        const int e = e0 + slot * kGramParts + part;
+        const int q = list[min(e, cnt - 1)];
+        const double *const yq = y + q * row_of;
+        double acc[2] = {0.0, 0.0};
+        for (int t = sub; t < len; t += 4 * kGramLanes) {
+          double a[4], b[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int tu = t + u * kGramLanes;
+            a[u] = tu < len ? x[tu * step] : 0.0;
+            b[u] = tu < len ? yq[tu * step] : 0.0;
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (t - sub + u * kGramLanes < len) acc[u & 1] = fma(a[u], b[u], acc[u & 1]);
+        }
+        double r = acc[0] + acc[1];
+#pragma unroll
+        for (int o = 1; o < kGramLanes; o <<= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+        if (e < cnt && sub == 0) {
+          blk[(int64_t)me * dim + q] = r;
+          if (SYM) blk[(int64_t)q * dim + me] = r;
+        }
+      }
+      __syncwarp();
+      if (lane < pending - cnt) list[lane] = list[lane + 32];
+      pending -= cnt;
+      __syncwarp();
     }
-    const double acc = dot_strided<false>(w + P.blk_base[g] + t, v + P.blk_base[g] + u, Pg, Q);
-    double *blk = sig + P.sig_off[g];
-    blk[(int64_t)t * Q + u] = acc;
-    if (SYM) blk[(int64_t)u * Q + t] = acc;
   }
 }
+
+constexpr int kTraceLanes = 8, kTraceAhead = 3;
 
 struct TraceTerm {
   const int64_t *row;
@@ -272,14 +323,18 @@ struct TraceTerm {
 };
 
 // Block partials of the trace of each term's operator against rho (LL, LR) or sigma (RR, RL):
-// blockIdx.y is the term, blockIdx.x a chunk of its runs / (RR, RL) positions.
+// blockIdx.y is the term, blockIdx.x a chunk of its runs / (RR, RL) positions, kTraceLanes lanes per run /
+// position, kTraceAhead elements of its operator row in flight in each.  Bound by the gathers: an element is
+// three dependent reads, and a thread per run spread each of a warp's reads over 32 lines.  64 terms of
+// Hubbard m=512: 22 us (a thread per run: 42 us; 16 or 4 lanes: 11 and 5 us more).
 __global__ void __launch_bounds__(kThreads) k_sb_trace(PairView P, SbStates S, const TraceTerm *__restrict__ terms,
                                                       const int *__restrict__ col, const double *__restrict__ val,
                                                       const double *__restrict__ rho0, const double *__restrict__ rho1,
                                                       const double *__restrict__ sig0, const double *__restrict__ sig1,
                                                       double *__restrict__ partials) {
   const TraceTerm t = terms[blockIdx.y];
-  const int first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  const int first = (blockIdx.x * blockDim.x + threadIdx.x) / kTraceLanes, stride = gridDim.x * blockDim.x / kTraceLanes;
+  const int sub = threadIdx.x % kTraceLanes;
   double acc = 0.0;
   if (t.pos == DG_SB_LL || t.pos == DG_SB_LR) {
     const double *__restrict__ rho = t.weight ? rho1 : rho0;
@@ -288,10 +343,22 @@ __global__ void __launch_bounds__(kThreads) k_sb_trace(PairView P, SbStates S, c
       const int a = P.run_ll[r], lr = P.run_lr[r];
       const int s = t.pos == DG_SB_LL ? a : lr;
       const double *__restrict__ rrow = rho + P.rho_off[g] + (int64_t)(r - r0) * Pg;
-      for (int64_t k = t.row[s]; k < t.row[s + 1]; ++k) {
-        const int c = col[k];
-        const int r2 = P.pair_run[t.pos == DG_SB_LL ? c * P.d + lr : a * P.d + c];
-        if (r2 >= r0 && r2 < r0 + Pg) acc += val[k] * rrow[r2 - r0];
+      const int64_t e = t.row[s + 1];
+      for (int64_t k = t.row[s] + sub; k < e; k += kTraceAhead * kTraceLanes) {
+        int r2[kTraceAhead];
+        double x[kTraceAhead], o[kTraceAhead];
+#pragma unroll
+        for (int u = 0; u < kTraceAhead; ++u) {
+          const int64_t ku = k + u * kTraceLanes;
+          const int c = ku < e ? col[ku] : -1;
+          o[u] = ku < e ? val[ku] : 0.0;
+          r2[u] = c >= 0 ? P.pair_run[t.pos == DG_SB_LL ? c * P.d + lr : a * P.d + c] : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < kTraceAhead; ++u) x[u] = r2[u] >= r0 && r2[u] < r0 + Pg ? rrow[r2[u] - r0] : 0.0;
+#pragma unroll
+        for (int u = 0; u < kTraceAhead; ++u)
+          if (r2[u] >= r0 && r2[u] < r0 + Pg) acc += o[u] * x[u];
       }
     }
   } else {
@@ -307,10 +374,22 @@ __global__ void __launch_bounds__(kThreads) k_sb_trace(PairView P, SbStates S, c
       const int s = t.pos == DG_SB_RR ? rr : rl;
       const double *__restrict__ srow = sig + P.sig_off[g] + (int64_t)tt * Q;
       const int *__restrict__ pos = P.rrrl_pos + g * tab;
-      for (int64_t k = t.row[s]; k < t.row[s + 1]; ++k) {
-        const int c = col[k];
-        const int t2 = pos[t.pos == DG_SB_RR ? c * P.d + rl : rr * P.d + c];
-        if (t2 >= 0) acc += val[k] * srow[t2];
+      const int64_t e = t.row[s + 1];
+      for (int64_t k = t.row[s] + sub; k < e; k += kTraceAhead * kTraceLanes) {
+        int t2[kTraceAhead];
+        double x[kTraceAhead], o[kTraceAhead];
+#pragma unroll
+        for (int u = 0; u < kTraceAhead; ++u) {
+          const int64_t ku = k + u * kTraceLanes;
+          const int c = ku < e ? col[ku] : -1;
+          o[u] = ku < e ? val[ku] : 0.0;
+          t2[u] = c >= 0 ? pos[t.pos == DG_SB_RR ? c * P.d + rl : rr * P.d + c] : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < kTraceAhead; ++u) x[u] = t2[u] >= 0 ? srow[t2[u]] : 0.0;
+#pragma unroll
+        for (int u = 0; u < kTraceAhead; ++u)
+          if (t2[u] >= 0) acc += o[u] * x[u];
       }
     }
   }
@@ -512,41 +591,32 @@ void launch_trace(const dg_sb_basis *b, const std::vector<SbTerm> &terms, const 
                   const double *w1, double *dout, cudaStream_t st) {
   const SbPairs &P = *b->pairs;
   const PairView pv = pair_view(P);
-  bool rows[2] = {false, false}, cols[2] = {false, false};
+  int need[2] = {0, 0};   // of each weight vector's density matrices
   std::vector<TraceTerm> tt;
   for (const SbTerm &t : terms) {
-    (t.pos == DG_SB_LL || t.pos == DG_SB_LR ? rows : cols)[t.weight] = true;
+    need[t.weight] |= t.pos == DG_SB_LL ? kNeedLL : t.pos == DG_SB_LR ? kNeedLR : t.pos == DG_SB_RR ? kNeedRR : kNeedRL;
     tt.push_back(TraceTerm{t.row, t.pos, t.weight});
   }
   DevBuf<double> rho[2], sig[2];
   const double *w[2] = {w0, w1};
   for (int k = 0; k < 2; ++k) {
-    const bool sym = w[k] == v;
-    if (rows[k]) {
-      rho[k].alloc(P.rho_off[P.B]);
-      const int64_t total = sym ? P.rho_tri[P.B] : P.rho_off[P.B];
-      if (sym)
-        k_gram_rows<true, false><<<(int)state_grid(total), kThreads, 0, st>>>(pv, w[k], v, rho[k].get());
-      else
-        k_gram_rows<false, false><<<(int)state_grid(total), kThreads, 0, st>>>(pv, w[k], v, rho[k].get());
-      count_launch();
-      DG_CUDA(cudaGetLastError());
-    }
-    if (cols[k]) {
-      sig[k].alloc(P.sig_off[P.B]);
-      const int64_t total = sym ? P.sig_tri[P.B] : P.sig_off[P.B];
-      if (sym)
-        k_gram_cols<true><<<(int)state_grid(total), kThreads, 0, st>>>(pv, w[k], v, sig[k].get());
-      else
-        k_gram_cols<false><<<(int)state_grid(total), kThreads, 0, st>>>(pv, w[k], v, sig[k].get());
-      count_launch();
-      DG_CUDA(cudaGetLastError());
-    }
+    if (!need[k]) continue;
+    if (need[k] & (kNeedLL | kNeedLR)) rho[k].alloc(P.rho_off[P.B]);
+    if (need[k] & (kNeedRR | kNeedRL)) sig[k].alloc(P.sig_off[P.B]);
+    const long warps = (need[k] & (kNeedLL | kNeedLR) ? P.R : 0) + (need[k] & (kNeedRR | kNeedRL) ? (long)P.q_off[P.B] : 0);
+    const int grid = (int)std::max(1L, std::min((warps * kGramParts + kGramWarps - 1) / kGramWarps, (long)sm_count() * 256));
+    if (w[k] == v)
+      k_gram_needed<true><<<grid, 32 * kGramWarps, 0, st>>>(pv, states_of(b), need[k], w[k], v, rho[k].get(), sig[k].get());
+    else
+      k_gram_needed<false><<<grid, 32 * kGramWarps, 0, st>>>(pv, states_of(b), need[k], w[k], v, rho[k].get(), sig[k].get());
+    count_launch();
+    DG_CUDA(cudaGetLastError());
   }
   DevBuf<TraceTerm> dterms(tt.size());
   DG_CUDA(cudaMemcpyAsync(dterms.get(), tt.data(), sizeof(TraceTerm) * tt.size(), cudaMemcpyHostToDevice, st));
   const int nt = (int)tt.size();
-  const int gx = (int)std::max(1L, std::min(8L, ((long)sm_count() * 4 + nt - 1) / nt));
+  const long items = std::max<long>(P.R, (long)P.q_off[P.B]), per = kThreads / kTraceLanes;
+  const int gx = (int)std::max(1L, std::min((items + per - 1) / per, ((long)sm_count() * 8 + nt - 1) / nt));
   DevBuf<double> partials((size_t)gx * nt);
   k_sb_trace<<<dim3(gx, nt), kThreads, 0, st>>>(pv, states_of(b), dterms.get(), ops->col.get(), ops->val.get(), rho[0].get(),
                                                 rho[1].get(), sig[0].get(), sig[1].get(), partials.get());
@@ -554,8 +624,7 @@ void launch_trace(const dg_sb_basis *b, const std::vector<SbTerm> &terms, const 
   DG_CUDA(cudaGetLastError());
   k_sb_expect_sum<<<nt, kThreads, 0, st>>>(partials.get(), gx, dout);
   count_launch();
-  DG_CUDA(cudaGetLastError());
-  DG_CUDA(cudaStreamSynchronize(st));   // dterms and the density matrices go out of scope
+  DG_CUDA(cudaGetLastError());   // (dterms and the density matrices are freed in stream order)
 }
 
 // out[t] for every term: sum over the states of w_{weight_t}[i] (O_t v)[i].  With one_sector (the
@@ -1102,7 +1171,7 @@ int dg_sb_density_matrix(const dg_sb_basis *b, const double *v, double *rho) {
       ob.alloc(total);
       dr = ob.get();
     }
-    k_gram_rows<true, true><<<(int)state_grid(P.rho_tri[P.B]), kThreads, 0, st>>>(pair_view(P), dv, dv, dr);
+    k_gram_rows<<<(int)state_grid(P.rho_tri[P.B]), kThreads, 0, st>>>(pair_view(P), dv, dr);
     count_launch();
     DG_CUDA(cudaGetLastError());
     if (!out_dev) DG_CUDA(cudaMemcpyAsync(rho, dr, sizeof(double) * total, cudaMemcpyDeviceToHost, st));
