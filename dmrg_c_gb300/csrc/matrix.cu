@@ -78,13 +78,15 @@ __global__ void k_full_counts(const int64_t *__restrict__ row, const int *__rest
     cnt[i] = (long long)(row[i + 1] - row[i]) + colcnt[i];
 }
 
-// Copy each lower row (strict part then the diagonal) to the front of its full row.
+// Copy each lower row (strict part then the diagonal) to the front of its full row, and set the
+// row's staging cursor: full offset less lower offset, the offset among the upper parts alone.
 __global__ void k_fill_lower(const int64_t *__restrict__ row, const int *__restrict__ col, const double *__restrict__ val,
-                             const int64_t *__restrict__ frow, int n, int *fcol, double *fval) {
+                             const int64_t *__restrict__ frow, int n, int *fcol, double *fval, unsigned long long *cursor) {
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
   for (int i = warp; i < n; i += nw) {
     int64_t b = row[i], len = row[i + 1] - b, f = frow[i];
+    if (lane == 0) cursor[i] = (unsigned long long)(f - b);
     for (int64_t k = lane; k < len; k += 32) {
       fcol[f + k] = col[b + k];
       fval[f + k] = val[b + k];
@@ -92,93 +94,120 @@ __global__ void k_fill_lower(const int64_t *__restrict__ row, const int *__restr
   }
 }
 
-// Scatter the transpose of the strict lower part into staging slots after each full
-// row's lower part (slot order within a row is arbitrary here; sorted afterwards).
+// An element of an upper part before it is sorted: one 16-byte store, one sector.
+struct __align__(16) Staged {
+  double v;
+  long long r;
+};
+
+// Scatter the transpose of the strict lower part, each column's elements one after another (in
+// arbitrary order; sorted afterwards).  Bound by the scattered atomics and stores: the
+// column's cursor is the position itself (with a counter, three more gathers an element found it) and
+// four elements a lane are in flight.  Hubbard m=512 (28 M elements): 435 us, before 640;
+// Kondo m=127 (1.5 M): 21 us, before 34.
 __global__ void __launch_bounds__(kThreads) k_fill_upper(const int64_t *__restrict__ row, const int *__restrict__ col,
-                                                        const double *__restrict__ val, const int64_t *__restrict__ frow, int n,
-                                                        int *fillctr, int *scol, double *sval) {
+                                                        const double *__restrict__ val, int n, unsigned long long *cursor,
+                                                        Staged *__restrict__ staged) {
+  constexpr int U = 4;
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
   for (int r = warp; r < n; r += nw) {
     const int64_t e = row[r + 1] - 1;
-    for (int64_t k = row[r] + lane; k < e; k += 32) {
-      const int c = col[k];
-      const int64_t lower_len = row[c + 1] - row[c];
-      const int64_t pos = frow[c] + lower_len + atomicAdd(fillctr + c, 1);
-      scol[pos] = r;
-      sval[pos] = val[k];
+    for (int64_t k0 = row[r] + lane; k0 < e; k0 += 32 * U) {
+      int c[U];
+      double v[U];
+      unsigned long long pos[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t k = k0 + 32 * u;
+        c[u] = k < e ? col[k] : -1;
+        v[u] = k < e ? val[k] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) pos[u] = c[u] >= 0 ? atomicAdd(cursor + c[u], 1ull) : 0ull;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (c[u] >= 0) staged[pos[u]] = Staged{v[u], (long long)r};
     }
   }
 }
 
-// Sort each row's upper segment by column (columns in a segment are distinct).  A warp per
-// row: segments of up to 64 entries rank every element against the others through register
-// shuffles (destination = rank); up to kSortCap entries are bitonic-sorted in shared memory
-// as keys (column << 32 | slot) with the values gathered by slot; longer segments fall back to
-// a rank count from memory.
-constexpr int kSortCap = 256;
-
-__global__ void __launch_bounds__(kThreads) k_rank_upper(const int64_t *__restrict__ row, const int64_t *__restrict__ frow, int n,
-                                                        const int *__restrict__ scol, const double *__restrict__ sval, int *fcol,
-                                                        double *fval) {
-  __shared__ unsigned long long keys[kWarps][kSortCap];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  unsigned long long *key = keys[wib];
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-  for (int i = warp; i < n; i += nw) {
-    const int64_t b = frow[i] + (row[i + 1] - row[i]), e = frow[i + 1];
-    const int m = (int)(e - b);
-    if (m <= 64) {
-      const int c0 = (lane < m) ? scol[b + lane] : INT_MAX;
-      const int c1 = (lane + 32 < m) ? scol[b + 32 + lane] : INT_MAX;
-      int r0 = 0, r1 = 0;
-      for (int u = 0; u < 32; ++u) {
-        const int v0 = __shfl_sync(0xffffffffu, c0, u), v1 = __shfl_sync(0xffffffffu, c1, u);
-        r0 += (v0 < c0) + (v1 < c0);
-        r1 += (v0 < c1) + (v1 < c1);
-      }
-      if (lane < m) {
-        fcol[b + r0] = c0;
-        fval[b + r0] = sval[b + lane];
-      }
-      if (lane + 32 < m) {
-        fcol[b + r1] = c1;
-        fval[b + r1] = sval[b + 32 + lane];
-      }
-    } else if (m <= kSortCap) {
-      int P = 1;
-      while (P < m) P <<= 1;
-      for (int t = lane; t < P; t += 32)
-        key[t] = (t < m) ? (((unsigned long long)(unsigned)scol[b + t] << 32) | (unsigned)t) : ~0ull;
-      __syncwarp();
-      for (int k = 2; k <= P; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-          for (int t = lane; t < P; t += 32) {
-            const int u = t ^ j;
-            if (u > t) {
-              const unsigned long long a = key[t], c = key[u];
-              if ((a > c) == ((t & k) == 0)) {
-                key[t] = c;
-                key[u] = a;
-              }
-            }
+// Ascending bitonic sort of 32 * R distinct keys held by a warp, element a * 32 + lane in key[a].
+template <class K, int R>
+__device__ __forceinline__ void warp_sort(K (&key)[R], int lane) {
+#pragma unroll
+  for (int k = 2; k <= 32 * R; k <<= 1) {
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) {
+#pragma unroll
+      for (int a = 0; a < R; ++a) {
+        if (j >= 32) {
+          const int b = a ^ (j >> 5);
+          if (b > a) {
+            const bool swap = (key[a] > key[b]) == (((a * 32) & k) == 0);
+            const K x = key[a], y = key[b];
+            key[a] = swap ? y : x;
+            key[b] = swap ? x : y;
           }
-          __syncwarp();
+        } else {
+          const K o = __shfl_xor_sync(0xffffffffu, key[a], j);
+          const bool low = ((lane & j) == 0) == (((a * 32 + lane) & k) == 0);
+          key[a] = low == (key[a] < o) ? key[a] : o;
         }
       }
-      for (int t = lane; t < m; t += 32) {
-        const unsigned long long kk = key[t];
-        fcol[b + t] = (int)(kk >> 32);
-        fval[b + t] = sval[b + (int)(kk & 0xffffffffu)];
-      }
-      __syncwarp();
+    }
+  }
+}
+
+// One upper part of m <= 32 * R staged elements to its place in the full row, by row index.
+template <class K, int R>
+__device__ __forceinline__ void place_upper(const Staged *__restrict__ in, int m, int *__restrict__ col, double *__restrict__ val, int lane) {
+  K key[R];
+#pragma unroll
+  for (int a = 0; a < R; ++a) key[a] = a * 32 + lane < m ? ((K)in[a * 32 + lane].r << 8) | (K)(a * 32 + lane) : ~(K)0;
+  warp_sort<K, R>(key, lane);
+#pragma unroll
+  for (int a = 0; a < R; ++a) {
+    const int t = a * 32 + lane;
+    if (t < m) {
+      col[t] = (int)(key[a] >> 8);
+      val[t] = in[(int)(key[a] & 0xff)].v;
+    }
+  }
+}
+
+// Sort each row's upper part by column.  A warp per row: up to kSortCap elements as keys (column and
+// slot) in registers, exchanged by shuffles; longer parts fall back to a rank count from memory.
+// K: 32-bit keys hold the columns of a matrix of up to 2^24 rows beside the 8 bits of the slot, 64-bit
+// ones any.  Bound by the exchanges (a sort of 128: 25 shuffled stages of 4 keys).  Hubbard m=512 (239 k
+// parts of 117): 327 us, before (keys of 8 bytes in shared memory, a rank count to 64) 1,000;
+// Kondo m=127 (50 k parts of 29): 20 us, before 36.
+constexpr int kSortCap = 256;
+
+template <class K>
+__global__ void __launch_bounds__(kThreads) k_rank_upper(const int64_t *__restrict__ row, const int64_t *__restrict__ frow, int n,
+                                                        const Staged *__restrict__ staged, int *fcol, double *fval) {
+  const int lane = threadIdx.x & 31;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  for (int i = warp; i < n; i += nw) {
+    const int64_t b = frow[i] + (row[i + 1] - row[i]);
+    const int64_t m = frow[i + 1] - b;
+    const Staged *const in = staged + (frow[i] - row[i]);
+    if (m <= 32) {
+      place_upper<K, 1>(in, (int)m, fcol + b, fval + b, lane);
+    } else if (m <= 64) {
+      place_upper<K, 2>(in, (int)m, fcol + b, fval + b, lane);
+    } else if (m <= 128) {
+      place_upper<K, 4>(in, (int)m, fcol + b, fval + b, lane);
+    } else if (m <= kSortCap) {
+      place_upper<K, 8>(in, (int)m, fcol + b, fval + b, lane);
     } else {
       for (int64_t t = lane; t < m; t += 32) {
-        const int c = scol[b + t];
+        const long long c = in[t].r;
         int64_t rank = 0;
-        for (int64_t u = 0; u < m; ++u) rank += (scol[b + u] < c);
-        fcol[b + rank] = c;
-        fval[b + rank] = sval[b + t];
+        for (int64_t u = 0; u < m; ++u) rank += in[u].r < c;
+        fcol[b + rank] = (int)c;
+        fval[b + rank] = in[t].v;
       }
     }
   }
@@ -250,42 +279,62 @@ __global__ void __launch_bounds__(kThreads) k_sell_widths(const int64_t *__restr
   }
 }
 
-// Column-major fill of each slice; padding: value 0, column = the slot's own row (or 0).
-template <class VT>
-__global__ void k_sell_fill(const int64_t *__restrict__ row, const int *__restrict__ col, const double *__restrict__ val,
-                            const int *__restrict__ perm, const int *__restrict__ width, const int64_t *__restrict__ off,
-                            int nslices, int *scol, VT *sval) {
-  const long slots = (long)nslices * kSellC;
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < slots; t += (long)gridDim.x * blockDim.x) {
-    const int sl = (int)(t / kSellC), l = (int)(t % kSellC);
-    const int r = perm[t];
+// Column-major fill of each slice; padding: value 0, column = the slot's own row (or 0).  A warp takes
+// tiles of 32 rows by kFillTile elements through shared memory, so that both the reads (along
+// the rows) and the writes (across them) are whole sectors; `parts` warps share a slice's tiles.
+// sval32 may be null.  Bound by memory: Hubbard m=512 (56 M elements) 225 us (6.0 TB/s), a thread per
+// row 0.38 ms; Kondo m=127 (3 M) 17 us, 30 us (too few threads).
+constexpr int kFillTile = 16, kFillWarps = 4;
+
+__global__ void __launch_bounds__(32 * kFillWarps) k_sell_fill(const int64_t *__restrict__ row, const int *__restrict__ col,
+                                                              const double *__restrict__ val, const int *__restrict__ perm,
+                                                              const int *__restrict__ width, const int64_t *__restrict__ off,
+                                                              int nslices, int parts, int *__restrict__ scol,
+                                                              double *__restrict__ sval, float *__restrict__ sval32) {
+  __shared__ int s_c[kFillWarps][kSellC][kFillTile + 1];
+  __shared__ double s_v[kFillWarps][kSellC][kFillTile + 1];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int half = lane / kFillTile, el = lane % kFillTile;   // a load covers two rows
+  const long nw = (long)gridDim.x * kFillWarps;
+  for (long it = (long)blockIdx.x * kFillWarps + wib; it < (long)nslices * parts; it += nw) {
+    const int sl = (int)(it / parts), part = (int)(it - (long)sl * parts);
+    const int r = perm[(long)sl * kSellC + lane];
     const int w = width[sl];
     const int64_t b = (r >= 0) ? row[r] : 0;
     const int len = (r >= 0) ? (int)(row[r + 1] - b) : 0;
-    const int64_t o = off[sl] + l;
-    int k = 0;
-    for (; k + 4 <= len; k += 4) {   // four loads in flight per lane
-      int c[4];
-      double v[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        c[u] = col[b + k + u];
-        v[u] = val[b + k + u];
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        scol[o + (int64_t)(k + u) * kSellC] = c[u];
-        sval[o + (int64_t)(k + u) * kSellC] = (VT)v[u];
-      }
-    }
-    for (; k < len; ++k) {
-      scol[o + (int64_t)k * kSellC] = col[b + k];
-      sval[o + (int64_t)k * kSellC] = (VT)val[b + k];
-    }
+    const int64_t o = off[sl] + lane;
     const int pad = r >= 0 ? r : 0;
-    for (; k < w; ++k) {
-      scol[o + (int64_t)k * kSellC] = pad;
-      sval[o + (int64_t)k * kSellC] = (VT)0;
+    for (int64_t k0 = (int64_t)part * kFillTile; k0 < w; k0 += (int64_t)parts * kFillTile) {
+#pragma unroll
+      for (int q0 = 0; q0 < kSellC / 2; q0 += 8) {
+        int c[8];
+        double v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int rr = 2 * (q0 + q) + half;
+          const int64_t bb = __shfl_sync(0xffffffffu, b, rr) + k0 + el;
+          const bool in = k0 + el < __shfl_sync(0xffffffffu, len, rr);
+          const int p = __shfl_sync(0xffffffffu, pad, rr);
+          c[q] = in ? col[bb] : p;
+          v[q] = in ? val[bb] : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          s_c[wib][2 * (q0 + q) + half][el] = c[q];
+          s_v[wib][2 * (q0 + q) + half][el] = v[q];
+        }
+      }
+      __syncwarp();
+      const int ke = (int)min((int64_t)kFillTile, w - k0);
+#pragma unroll 4
+      for (int k = 0; k < ke; ++k) {
+        const int64_t e = o + (k0 + k) * kSellC;
+        const double v = s_v[wib][lane][k];
+        scol[e] = s_c[wib][lane][k];
+        sval[e] = v;
+        if (sval32) sval32[e] = (float)v;
+      }
+      __syncwarp();
     }
   }
 }
@@ -476,12 +525,12 @@ void build_sell(dg_matrix *m, cudaStream_t st, int window) {
     m->s_d16.release();
     m->s_chk.release();
     m->s_choff.release();
-    k_sell_fill<double><<<g, kThreads, 0, st>>>(m->row.get(), m->col.get(), m->val.get(), m->s_perm.get(), m->s_width.get(),
-                                                m->s_off.get(), nslices, m->s_col.get(), m->s_val.get()); ::dg::count_launch();
-    if (m->has32) {
-      k_sell_fill<float><<<g, kThreads, 0, st>>>(m->row.get(), m->col.get(), m->val.get(), m->s_perm.get(), m->s_width.get(),
-                                                 m->s_off.get(), nslices, m->s_col.get(), m->s_val32.get()); ::dg::count_launch();
-    }
+    // warps a slice: one per tile of an average slice, up to four
+    const int parts = (int)std::max(1L, std::min(4L, (long)(total / ((int64_t)nslots * kFillTile))));
+    const long need = ((long)nslices * parts + kFillWarps - 1) / kFillWarps;
+    k_sell_fill<<<(int)std::min(need, (long)sm_count() * 64), 32 * kFillWarps, 0, st>>>(
+        m->row.get(), m->col.get(), m->val.get(), m->s_perm.get(), m->s_width.get(), m->s_off.get(), nslices, parts, m->s_col.get(),
+        m->s_val.get(), m->has32 ? m->s_val32.get() : nullptr); ::dg::count_launch();
     if (sell_uses_deltas(m->sell_variant)) m->sell_variant = V_U8;
     if (sell_uses_deltas(m->sell_variant32)) m->sell_variant32 = V_U8;
   }
@@ -583,10 +632,9 @@ dg_matrix *matrix_from_device(int n, long nnz_in, const long *row_d, const int *
       DG_CUDA(cudaMemcpyAsync(m->col.get(), col_d, sizeof(int) * nnz_in, cudaMemcpyDeviceToDevice, st));
       DG_CUDA(cudaMemcpyAsync(m->val.get(), val_d, sizeof(double) * nnz_in, cudaMemcpyDeviceToDevice, st));
     } else {
-      DevBuf<int> colcnt(n), fillctr(n);
+      DevBuf<int> colcnt(n);
       DevBuf<long long> cnt(n), tmp((n + kScanTile - 1) / kScanTile + 2);
       DG_CUDA(cudaMemsetAsync(colcnt.get(), 0, sizeof(int) * n, st));
-      DG_CUDA(cudaMemsetAsync(fillctr.get(), 0, sizeof(int) * n, st));
       k_count_upper<<<g, kThreads, 0, st>>>(row, col_d, n, colcnt.get()); ::dg::count_launch();
       k_full_counts<<<g, kThreads, 0, st>>>(row, colcnt.get(), n, cnt.get()); ::dg::count_launch();
       m->row.alloc(n + 1);
@@ -598,12 +646,15 @@ dg_matrix *matrix_from_device(int n, long nnz_in, const long *row_d, const int *
       m->nnz = total;
       m->col.alloc(total);
       m->val.alloc(total);
-      DG_CUDA(cudaMemsetAsync(m->col.get(), 0, sizeof(int) * total, st));
-      DevBuf<int> scol(total);
-      DevBuf<double> sval(total);
-      k_fill_lower<<<gw, kThreads, 0, st>>>(row, col_d, val_d, m->row.get(), n, m->col.get(), m->val.get()); ::dg::count_launch();
-      k_fill_upper<<<gw, kThreads, 0, st>>>(row, col_d, val_d, m->row.get(), n, fillctr.get(), scol.get(), sval.get()); ::dg::count_launch();
-      k_rank_upper<<<gw, kThreads, 0, st>>>(row, m->row.get(), n, scol.get(), sval.get(), m->col.get(), m->val.get()); ::dg::count_launch();
+      DevBuf<unsigned long long> cursor(n);
+      DevBuf<Staged> staged(nnz_in - n);   // the upper parts
+      k_fill_lower<<<gw, kThreads, 0, st>>>(row, col_d, val_d, m->row.get(), n, m->col.get(), m->val.get(), cursor.get()); ::dg::count_launch();
+      k_fill_upper<<<gw, kThreads, 0, st>>>(row, col_d, val_d, n, cursor.get(), staged.get()); ::dg::count_launch();
+      if (n <= 1 << 24)
+        k_rank_upper<unsigned><<<gw, kThreads, 0, st>>>(row, m->row.get(), n, staged.get(), m->col.get(), m->val.get());
+      else
+        k_rank_upper<unsigned long long><<<gw, kThreads, 0, st>>>(row, m->row.get(), n, staged.get(), m->col.get(), m->val.get());
+      ::dg::count_launch();
       DG_CUDA(cudaGetLastError());
       DG_CUDA(cudaStreamSynchronize(st));
     }
