@@ -28,6 +28,7 @@
 #include "apply.cuh"
 #include "sell.cuh"
 #include "common.cuh"
+#include "cg_cluster.cuh"
 #include "dense.cuh"
 #include "tridiag.h"
 
@@ -988,11 +989,20 @@ IterResult cg_core(const Opl &op, double sigma, const double *b_dev, double *x_d
   op.apply(x_dev, Scale::norm2(&S->xn2), sigma, (const int *)nullptr, EpiCgInit{b_dev, xs.get(), r.get(), p.get(), S}, slot, st);
   DG_CUDA(cudaMemcpyAsync(x_dev, xs.get(), sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
   if (spmv_count) ++*spmv_count;
-  const int chunk = 8;
+  // small systems: a chunk of iterations is one kernel on one cluster
+  const dg_matrix *small = op.matrix() && cg_cluster_takes(op.matrix()) ? op.matrix() : nullptr;
+  const int chunk = small ? 32 : 8;
   int enq = 0;   // last iteration enqueued
   const int pgrid = op.grid();
   double *up = ws.partials2.get();
   auto enqueue_to = [&](int last) {
+    if (small) {
+      if (last > enq)
+        launch_cg_cluster(small, CgCluster{n, nullptr, nullptr, nullptr, sigma, x_dev, r.get(), p.get(), S, ws.prog.d, enq + 1, last,
+                                           max_step, acc}, st);
+      enq = std::max(enq, last);
+      return;
+    }
     for (int it = enq + 1; it <= last; ++it) {
       op.apply(p.get(), Scale{}, sigma, &S->done, EpiCgDot{y.get()}, slot, st);
       launch_pdl(ws.uthreads == kThreads ? k_cg_update<kThreads> : k_cg_update<512>, ws.ugrid, ws.uthreads, st, n,
