@@ -340,20 +340,23 @@ __global__ void __launch_bounds__(32 * kFillWarps) k_sell_fill(const int64_t *__
 }
 
 // Bridges each row needs for the 16-bit delta stream: (gap - 1) / 65,535 zero elements for a gap
-// between neighbouring columns; blen[r] = length + bridges.  A warp per row.  stats[0] counts
-// rows whose columns decrease (then there is no delta stream) or whose laid-out length would
-// overflow an int; stats[1] sums the bridges (one atomic per block).
+// between neighbouring columns; blen[r] = length + bridges.  G lanes per row: a warp for the superblocks,
+// eight lanes for rows of a few elements (ED Hamiltonians, 13 a row: 48 us against 110 with a
+// warp a row).  stats[0] counts rows whose columns decrease (then there is no delta stream) or
+// whose laid-out length would overflow an int; stats[1] sums the bridges (one atomic per block).
+template <int G>
 __global__ void __launch_bounds__(kThreads) k_row_bridges(const int64_t *__restrict__ row, const int *__restrict__ col, int n,
                                                          int *blen, unsigned long long *stats) {
   __shared__ unsigned long long s_br[kWarps], s_bad[kWarps];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, sub = threadIdx.x % G;
+  const long group = (blockIdx.x * (long)blockDim.x + threadIdx.x) / G, ng = gridDim.x * (long)blockDim.x / G;
   unsigned long long br_w = 0, bad_w = 0;
-  for (int r = warp; r < n; r += nw) {
-    const int64_t b = row[r], len = row[r + 1] - b;
+  for (long r0 = group - lane / G; r0 < n; r0 += ng) {   // (the warp's first row: its lanes stay together)
+    const long r = r0 + lane / G;
+    const int64_t b = r < n ? row[r] : 0, len = r < n ? row[r + 1] - b : 0;
     unsigned long long br = 0;
     bool dec = false;
-    for (int64_t k = 1 + lane; k < len; k += 32) {
+    for (int64_t k = 1 + sub; k < len; k += G) {
       const long long gap = (long long)col[b + k] - col[b + k - 1];
       if (gap < 0)
         dec = true;
@@ -361,14 +364,20 @@ __global__ void __launch_bounds__(kThreads) k_row_bridges(const int64_t *__restr
         br += (unsigned long long)((gap - 1) / kSellBridge);
     }
 #pragma unroll
-    for (int o = 16; o; o >>= 1) br += __shfl_xor_sync(0xffffffffu, br, o);
-    dec = __any_sync(0xffffffffu, dec);
-    const unsigned long long laid = (unsigned long long)len + br;
-    if (lane == 0) {
+    for (int o = G / 2; o; o >>= 1) br += __shfl_xor_sync(0xffffffffu, br, o);
+    const unsigned decs = __ballot_sync(0xffffffffu, dec);
+    if (sub == 0 && r < n) {
+      const bool any = (decs >> (lane & ~(G - 1))) & (G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u);
+      const unsigned long long laid = (unsigned long long)len + br;
       blen[r] = laid > 0x7fffffffull ? 0x7fffffff : (int)laid;
       br_w += br;
-      bad_w += (dec || laid > 0x7fffffffull) ? 1 : 0;
+      bad_w += (any || laid > 0x7fffffffull) ? 1 : 0;
     }
+  }
+#pragma unroll
+  for (int o = 16; o >= G; o >>= 1) {   // the warp's rows' first lanes
+    br_w += __shfl_xor_sync(0xffffffffu, br_w, o);
+    bad_w += __shfl_xor_sync(0xffffffffu, bad_w, o);
   }
   if (lane == 0) {
     s_br[wib] = br_w;
@@ -483,7 +492,9 @@ void build_sell(dg_matrix *m, cudaStream_t st, int window) {
     blen.alloc(n);
     DevBuf<unsigned long long> stats(2);
     DG_CUDA(cudaMemsetAsync(stats.get(), 0, 2 * sizeof(unsigned long long), st));
-    k_row_bridges<<<warp_grid(n), kThreads, 0, st>>>(m->row.get(), m->col.get(), n, blen.get(), stats.get()); ::dg::count_launch();
+    const bool shorter = m->nnz < 24L * n;
+    auto bridges = shorter ? k_row_bridges<8> : k_row_bridges<32>;
+    bridges<<<warp_grid(shorter ? (n + 3) / 4 : n), kThreads, 0, st>>>(m->row.get(), m->col.get(), n, blen.get(), stats.get()); ::dg::count_launch();
     unsigned long long h[2] = {0, 0};
     DG_CUDA(cudaMemcpyAsync(h, stats.get(), sizeof(h), cudaMemcpyDeviceToHost, st));
     DG_CUDA(cudaStreamSynchronize(st));
