@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(kThreads) k_mx_update(float *__restrict__ V, l
   const float *vb = V + (long)b * ldv;
   const float *vp = (b > 0) ? V + (long)(b - 1) * ldv : vb;
   float *vn = V + (long)(b + 1) * ldv;
-  // first element's operands in flight before the partial sums (see k_lz_update)
+  // first element's operands in flight before the partial sums (see k_lz_step)
   const int i0 = blockIdx.x * kThreads + threadIdx.x, stride = gridDim.x * kThreads;
   float y0 = 0.0f, b0 = 0.0f, q0 = 0.0f;
   if (i0 < n) {

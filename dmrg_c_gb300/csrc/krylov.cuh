@@ -58,9 +58,9 @@ struct Progress {
   volatile int done;
 };
 
-// Launch shape of the step kernels (k_lz_step, k_cg_update, k_cg_direction).  Every block sums the product's partials (up to ~1,900 a
-// sum) before its elements, and on GB300 a warp-wide FP64 add holds an SM's FP64 pipe for ~19
-// cycles: with four blocks a SM those sums were most of the kernels' time at 238 k elements (9.6 us
+// Launch shape of the step kernels (k_lz_step, k_cg_update, k_cg_direction).  Every block sums the
+// product's partials (up to ~1,900 a sum) before its elements, and on GB300 a warp-wide FP64 add
+// holds an SM's FP64 pipe for ~19 cycles: with four blocks a SM those sums were most of the kernels' time at 238 k elements (9.6 us
 // for 2 us of traffic).  So large vectors get one block of 512 threads a SM; small ones, where the
 // elements' own FP64 work counts, one thread an element.
 constexpr int kStepAhead = 2;   // elements a thread loads before the partial sums

@@ -9,7 +9,7 @@ __global__ void __launch_bounds__(kThreads) k_refine32_update(int n, const float
                                                              int pcount, const float2 *gpp, int gcount, float2 *up) {
   pdl_wait();
   if (*((volatile const int *)&S->done)) return;
-  // first element's operands in flight before the partial sums (see k_lz_update)
+  // first element's operands in flight before the partial sums (see k_lz_step)
   const int i0 = blockIdx.x * kThreads + threadIdx.x, stride = gridDim.x * kThreads;
   float t0 = 0.0f, f0 = 0.0f, r0 = 0.0f, q0 = 0.0f, s0 = 0.0f;
   if (i0 < n) {
@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(kThreads) k_refine32_direction(int n, const fl
                                                                 const float2 *up, int ucount, float2 *gout, Progress *prog) {
   pdl_wait();
   if (*((volatile const int *)&S->done)) return;
-  // first element's operands in flight before the partial sums (see k_lz_update)
+  // first element's operands in flight before the partial sums (see k_lz_step)
   const int i0 = blockIdx.x * kThreads + threadIdx.x, stride = gridDim.x * kThreads;
   float r0 = 0.0f, p0 = 0.0f, g0 = 0.0f;
   if (i0 < n) {

@@ -197,12 +197,12 @@ int dg_matrix_set_sell_shape(dg_matrix *m, int warps_per_slice, int grid);
  * by bulk copies (with more warps per slice it runs variant 1); 5: groups of 8 on the 16-bit
  * column-delta stream (warps of a slice take whole 32-element chunks); 6: variant 4 on the
  * delta stream (with more warps per slice it runs variant 5).  Variants 5 and 6 need the delta
- * stream (dg_matrix_sell_deltas; DG_ERR_ARG otherwise).  The FP64 product's default follows
- * the warps per slice (3 for 1-2 warps, 2 for 4-8), the FP32 (mixed) product's is 1; this call
- * sets both. */
+ * stream (dg_matrix_sell_deltas; DG_ERR_ARG otherwise).  The FP64 product's default is 3, or
+ * 2 for short rows (< 24 stored a row) and for 4-8 warps a slice of >= 32 elements each; the FP32
+ * (mixed) product's is 1, or 5 with the delta stream; this call sets both. */
 int dg_matrix_set_sell_variant(dg_matrix *m, int variant);
-/* Warps per slice and variant of the FP32 (mixed-precision) product alone; it keeps the grid
- * of dg_matrix_set_sell_shape. */
+/* Warps per slice and variant of the FP32 (mixed-precision) product alone; its grid stays (the
+ * default's, or that of dg_matrix_set_sell_shape, which sets both products). */
 int dg_matrix_set_sell_mixed(dg_matrix *m, int warps_per_slice, int variant);
 /* *present = 1 if the sliced-ELL copy carries the 16-bit column-delta stream (built for
  * matrices with FP32 values (DG_VALUES_F32 / DG_VALUES_BOTH) of at least 4M stored elements
