@@ -261,7 +261,10 @@ __global__ void k_mx_ritz_coef(const double *__restrict__ s, const double *__res
 
 // The FP32 Krylov basis combined on the FP32 pipes: with FP64 coefficients each (element,
 // vector) term took three FP64 instructions (a 49-vector combination of the XXZ L=22 basis
-// ran 221 us, FP64-issue bound); here the FP64 work is one conversion per element.
+// ran 221 us, FP64-issue bound); here the FP64 work is one conversion per element.  Bound by the
+// bytes in flight: kRitzAhead loads a thread (78 vectors of Hubbard L=12, 266 MB: 87 us, eight loads 170).
+constexpr int kRitzAhead = 16;
+
 __global__ void __launch_bounds__(kThreads) k_mx_ritz(const float *__restrict__ V, long ldv, int k, const float2 *__restrict__ cp,
                                                      double *__restrict__ out, int n, Norm2 *r2, RedSlot slot) {
   extern __shared__ float2 cs[];   // k entries
@@ -271,12 +274,12 @@ __global__ void __launch_bounds__(kThreads) k_mx_ritz(const float *__restrict__ 
   for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
     AccDot2 t;
     int j = 0;
-    for (; j + 8 <= k; j += 8) {   // eight loads in flight per thread
-      float v[8];
+    for (; j + kRitzAhead <= k; j += kRitzAhead) {
+      float v[kRitzAhead];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = __ldg(V + (long)(j + u) * ldv + i);
+      for (int u = 0; u < kRitzAhead; ++u) v[u] = __ldg(V + (long)(j + u) * ldv + i);
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
+      for (int u = 0; u < kRitzAhead; ++u) {
         t.add(cs[j + u].x, v[u]);
         t.add(cs[j + u].y, v[u]);
       }
