@@ -866,6 +866,7 @@ struct BatchLanczosImpl {
             admit(*in, st);
           } catch (const Error &e) {
             ok = false;
+            cudaStreamSynchronize(st);   // its own mirrors, if it has any, go back when it is destroyed
             release(*in, st);
             finish(*in, e.code, last_error(), nullptr, nullptr, 0.0, 0, false);
           }

@@ -87,7 +87,9 @@ void *pool_alloc(size_t bytes, cudaStream_t st);
 void pool_free(void *p, cudaStream_t st);
 
 // Mapped pinned host memory is kept in a bounded list of blocks, shared by all threads, for the
-// same reason (cudaHostAlloc / cudaFreeHost cost far more than one solver step).
+// same reason (cudaHostAlloc / cudaFreeHost cost far more than one solver step).  A block is returned
+// when the calling thread's stream has drained, or while an exception unwinds (the list then waits
+// for that stream before it hands the block out again).
 void *mapped_acquire(size_t bytes, size_t *got);
 void mapped_return(void *h, size_t bytes);
 

@@ -2,6 +2,7 @@
 #include <atomic>
 #include <chrono>
 #include <cstdarg>
+#include <exception>
 #include <mutex>
 
 #include "common.cuh"
@@ -40,7 +41,19 @@ void require_device() {
 // process had ever used stayed in the driver's list that a stream-ordered allocation walks:
 // after ~100 batched calls of 9 threads each a resident expectation value took 10.5 ms instead
 // of 0.25 ms and a batched solve of 24 chains 76 ms instead of 27.
+// A call that gave up (a wait that ran out, an allocation that failed) leaves work queued on its
+// stream: such a stream stays in the list, and is passed over until the work has finished, so that
+// no other thread waits behind it.
 namespace {
+// Queries of streams and events that another thread's stream capture must not see.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() {
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (cudaPeekAtLastError() == cudaErrorNotReady) cudaGetLastError();   // a query's, no error of the caller's
+  }
+};
 constexpr int kMaxPoolDevices = 64;
 constexpr size_t kKeptStreams = 64;   // idle streams kept per device; more are destroyed
 struct IdleStreams {
@@ -57,7 +70,6 @@ struct ThreadStream {
   int dev = -1;
   void give_back() {
     if (!s) return;
-    // work still queued on it stays in order before the next owner's
     bool kept = false;
     if (dev >= 0 && dev < kMaxPoolDevices) {
       IdleStreams &is = idle_streams();
@@ -74,9 +86,14 @@ struct ThreadStream {
     if (device >= 0 && device < kMaxPoolDevices) {
       IdleStreams &is = idle_streams();
       std::lock_guard<std::mutex> lk(is.mu);
-      if (!is.idle[device].empty()) {
-        s = is.idle[device].back();
-        is.idle[device].pop_back();
+      std::vector<cudaStream_t> &idle = is.idle[device];
+      if (!idle.empty()) {
+        RelaxedCapture relaxed;
+        for (size_t i = idle.size(); i-- > 0 && !s;)
+          if (cudaStreamQuery(idle[i]) == cudaSuccess) {
+            s = idle[i];
+            idle.erase(idle.begin() + (long)i);
+          }
       }
     }
     if (!s) DG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
@@ -171,16 +188,33 @@ void pool_free(void *p, cudaStream_t st) {
 // One list for the process: a block returned by one thread serves the next solve of any thread
 // (a worker thread of the batched form lives for one call; with a list per thread it allocated
 // its blocks anew and freed them at its end, and freeing pinned memory waits for the device).
+// A solve returns its blocks after its stream has drained, except when an error unwinds it: kernels
+// it has queued may then still write them.  Such a block waits behind an event recorded on the
+// stream and is handed out again only after that.
 namespace {
 struct MappedBlock {
   void *h;
   size_t bytes;
+  cudaEvent_t written = nullptr;   // the block's last writers (blocks in `busy`)
 };
 constexpr size_t kKeptBlocks = 256, kKeptBlockBytes = size_t(64) << 20;   // more are freed
 struct MappedList {
   std::mutex mu;
-  std::vector<MappedBlock> idle;
-  size_t bytes = 0;
+  std::vector<MappedBlock> idle, busy;
+  size_t bytes = 0;   // of both
+  bool room(size_t more) const { return idle.size() + busy.size() < kKeptBlocks && bytes + more <= kKeptBlockBytes; }
+  // Blocks whose writers have finished become idle.
+  void collect() {
+    if (busy.empty()) return;
+    RelaxedCapture relaxed;
+    for (size_t i = busy.size(); i-- > 0;)
+      if (cudaEventQuery(busy[i].written) == cudaSuccess) {
+        cudaEventDestroy(busy[i].written);
+        idle.push_back(MappedBlock{busy[i].h, busy[i].bytes});
+        busy[i] = busy.back();
+        busy.pop_back();
+      }
+  }
 };
 MappedList &mapped_list() {   // never destroyed, as idle_streams()
   static MappedList *l = new MappedList();
@@ -194,6 +228,7 @@ void *mapped_acquire(size_t bytes, size_t *got) {
   {
     MappedList &l = mapped_list();
     std::lock_guard<std::mutex> lk(l.mu);
+    l.collect();
     size_t best = l.idle.size();   // the smallest block that fits
     for (size_t i = 0; i < l.idle.size(); ++i)
       if (l.idle[i].bytes >= want && (best == l.idle.size() || l.idle[i].bytes < l.idle[best].bytes)) best = i;
@@ -212,18 +247,37 @@ void *mapped_acquire(size_t bytes, size_t *got) {
   return h;
 }
 
+namespace {
+// An event behind everything this thread has queued; null if it cannot be had.
+cudaEvent_t event_behind_stream() {
+  cudaEvent_t ev = nullptr;
+  try {
+    cudaStream_t st = stream();
+    if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return nullptr;
+    if (cudaEventRecord(ev, st) == cudaSuccess) return ev;
+    cudaEventDestroy(ev);
+  } catch (const Error &) {
+  }
+  return nullptr;
+}
+}  // namespace
+
 void mapped_return(void *h, size_t bytes) {
   if (!h) return;
+  const bool unwinding = std::uncaught_exceptions() > 0;
+  const cudaEvent_t written = unwinding ? event_behind_stream() : nullptr;
+  if (unwinding && !written) return;   // nothing says when its writers end: given up
+  MappedList &l = mapped_list();
   {
-    MappedList &l = mapped_list();
     std::lock_guard<std::mutex> lk(l.mu);
-    if (l.idle.size() < kKeptBlocks && l.bytes + bytes <= kKeptBlockBytes) {
-      l.idle.push_back(MappedBlock{h, bytes});
+    if (l.room(bytes)) {
+      (unwinding ? l.busy : l.idle).push_back(MappedBlock{h, bytes, written});
       l.bytes += bytes;
       return;
     }
   }
-  cudaFreeHost(h);
+  if (written) cudaEventDestroy(written);
+  cudaFreeHost(h);   // (waits for the device)
 }
 
 int sm_count() {
