@@ -406,6 +406,9 @@ __global__ void __launch_bounds__(threads, threads == kThreads ? 5 : 1) k_jacobi
       if (any) cur ^= 1;
     }
   }
+  // The last rounds of the last sweep may have been idle ones, without a barrier: no CTA leaves while
+  // another still reads its rows.
+  cluster.sync();
   const double *A = mine + cur * slab;
   for (int i = tid; i < nloc; i += threads) Wg[b.woff + r0 + i] = A[(int64_t)i * n + r0 + i];
   for (int64_t e = tid; e < (int64_t)nloc * n; e += threads) Vg[b.off + (int64_t)r0 * n + e] = V[e];
