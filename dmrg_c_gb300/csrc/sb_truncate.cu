@@ -584,7 +584,7 @@ DMRG_SYSTEM_INFO *system_info(int nq, const int *const *qn, DMRG_BASIS *B, const
         // 31.7 ms, 122 9.7 / 10.1, 96 7.6 / 7.2, 65 4.1 / 3.7; 8 CTAs: 40 1.50 / 1.34, 14 0.49 / 0.44.
         const int workers = alone && mn >= kJacobiAhead && (gmem || smem_for(cs - 1, mn) <= kJacobiSmem) ? cs - 1 : cs;
         const size_t need = gmem ? 0 : smem_for(workers, mn);
-        cfg.dynamicSmemBytes = need;
+        cfg.dynamicSmemBytes = alone && mn >= kJacobiAhead ? std::max(need, kJacobiAlone) : need;   // (one CTA a SM)
         cfg.stream = st;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -601,7 +601,6 @@ DMRG_SYSTEM_INFO *system_info(int nq, const int *const *qn, DMRG_BASIS *B, const
           cs = 8;   // try the portable size
           continue;
         }
-        if (alone && mn >= kJacobiAhead) cfg.dynamicSmemBytes = std::max(need, kJacobiAlone);   // one CTA a SM
         const int64_t gstride = 3 * (int64_t)((mn + workers - 1) / workers) * mn;
         if (gmem) gwork.alloc((size_t)count * cs * gstride);
         DG_CUDA(cudaLaunchKernelEx(&cfg, kernel, (const EigBlk *)(deb.get() + first), (const double *)dA.get(), dV.get(), dW.get(),
