@@ -130,14 +130,13 @@ void launch_cg_cluster(const dg_matrix *m, CgCluster a, cudaStream_t st) {
   a.col = m->col.get();
   a.val = m->val.get();
   auto kernel = m->nnz > 16L * a.n ? k_cg_cluster<8> : k_cg_cluster<4>;
-  // clusters of 16 need an opt-in; a device that refuses it gets 8
-  const bool wide = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-  cudaGetLastError();
+  constexpr int kSmem = (int)sizeof(double) * (kCgClusterN + 3 * (kCgClusterN / 8));
+  DG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+  // a device that runs no cluster of 16 gets 8
+  const bool wide = runs_cluster16((const void *)kernel, kCgThreads, kSmem);
   int cs = 1;
   while (cs < (wide ? 16 : 8) && cs * 32 < a.n) cs <<= 1;
   const int rows = (a.n + cs - 1) / cs;
-  constexpr int kSmem = (int)sizeof(double) * (kCgClusterN + 3 * (kCgClusterN / 8));
-  DG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
   cudaLaunchConfig_t cfg;
   std::memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((unsigned)cs);

@@ -179,6 +179,11 @@ void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t st
   launch_pdl_smem(kernel, grid, block, 0, st, args...);
 }
 
+// Whether the current device runs a cluster of 16 CTAs (a non-portable size: it depends on the SMs a GPC
+// has left) of the kernel with this many threads and bytes of dynamic shared memory, which the caller has
+// allowed it.  Asked of the driver once per device and kernel.
+bool runs_cluster16(const void *kernel, int threads, size_t smem);
+
 // Is p a device (or managed) pointer?  Plain host memory (malloc) is "unregistered".
 bool is_device_ptr(const void *p);
 // Is p device memory the host cannot read (not managed, not host)?

@@ -160,10 +160,10 @@ bool launch_dense_step(const dg_matrix *m, DenseStep a, cudaStream_t st) {
   a.val = m->val.get();
   if (a.n > kDenseMaxN) return false;
   auto kernel = m->nnz > 16L * a.n ? k_dense_step<8> : k_dense_step<4>;
-  // clusters of 16 need an opt-in; a device that refuses it runs systems of up to 8 CTAs' rows
-  DG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kDenseFixedBytes + kDenseBasisBytes)));
-  const bool wide = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-  cudaGetLastError();
+  constexpr size_t kMost = kDenseFixedBytes + kDenseBasisBytes;
+  DG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
+  // a device that runs no cluster of 16 takes systems of up to 8 CTAs' rows
+  const bool wide = runs_cluster16((const void *)kernel, kThreads, kMost);
   // about 32 rows a CTA, so that a row's four threads and the barrier's cost both count little
   int cs = 1;
   while (cs < 16 && cs * 32 < a.n) cs <<= 1;

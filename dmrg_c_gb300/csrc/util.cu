@@ -3,7 +3,9 @@
 #include <chrono>
 #include <cstdarg>
 #include <exception>
+#include <map>
 #include <mutex>
+#include <utility>
 
 #include "common.cuh"
 
@@ -296,6 +298,33 @@ int vector_grid(long n) {
   long cap = (long)sm_count() * 4;
   if (need < 1) need = 1;
   return (int)(need < cap ? need : cap);
+}
+
+bool runs_cluster16(const void *kernel, int threads, size_t smem) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void *>, bool> known;
+  int dev = 0;
+  DG_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(mu);
+  const auto it = known.find({dev, kernel});
+  if (it != known.end()) return it->second;
+  cudaLaunchConfig_t cfg;
+  std::memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(16);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 16;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                  cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters >= 1;
+  if (!ok) cudaGetLastError();   // refused, not an error
+  return known[{dev, kernel}] = ok;
 }
 
 bool is_device_ptr(const void *p) {
