@@ -455,13 +455,24 @@ void launch_validate(const int64_t *row, const int *col, int n, long nnz, int lo
   k_validate<<<warp_grid(n), kThreads, 0, st>>>(row, col, n, nnz, lower, bad); ::dg::count_launch();
 }
 
-// Blocks a SM of the sliced-ELL grids: of the FP64 product's pipelined form, and of the others.
+// Blocks a SM of the sliced-ELL grids: of the FP64 product's pipelined form, and of the others.  The
+// pipelined form runs three blocks a SM (78 registers): one wave of blocks that walk the slices
+// beats several (Hubbard m=512 126 against 130 us, Kondo m=127 16.9 against 17.4) and leaves a
+// quarter of the reduction partials for the next kernel to sum.  The FP32 product is slower on one wave, and
+// its sums would be grouped otherwise.
 constexpr int kSellBpsPipe = 3, kSellBps = 16;
 
 static int sell_grid_for(const dg_matrix *m, int ws, int bps) {
   const int groups = kWarps / ws;
   const long need = (m->nslices + groups - 1) / groups;
   return (int)std::max(1L, std::min(need, (long)sm_count() * bps));
+}
+static int sell_bps(int variant) { return variant == V_PIPE8 ? kSellBpsPipe : kSellBps; }
+// The default grid of each product: for its own warps per slice and, FP64, its variant.
+static void default_sell_grids(dg_matrix *m) {
+  m->sell_grid = sell_grid_for(m, m->sell_ws, sell_bps(m->sell_variant));
+  m->sell_grid32 = sell_grid_for(m, m->sell_ws32, kSellBps);
+  m->sell_grid_given = false;
 }
 
 void build_sell(dg_matrix *m, cudaStream_t st, int window) {
@@ -549,9 +560,7 @@ void build_sell(dg_matrix *m, cudaStream_t st, int window) {
   const SellShape f64 = choose_sell_shape(n, nslices, total, false), f32 = choose_sell_shape(n, nslices, total, true);
   m->sell_ws = f64.ws;
   m->sell_variant = f64.variant;
-  m->sell_grid = f64.grid;
   m->sell_ws32 = f32.ws;
-  m->sell_grid32 = f32.grid;
   // The FP32 product on the delta stream (6 bytes an element instead of 8): on the Hubbard m=512
   // superblock of a DMRG sweep (238 k rows of 236 stored elements) 8-element groups with the next chunk prefetched into L2 took
   // 79 us at one warp per slice and 81 at two, against 92 us for the 32-bit columns.  One warp a
@@ -559,13 +568,11 @@ void build_sell(dg_matrix *m, cudaStream_t st, int window) {
   // gains nothing from the deltas and keeps its variant.
   if (m->has_d16()) {
     m->sell_variant32 = V_D8;
-    if (m->sell_ws32 <= 2 && (long)nslices >= 24L * sm_count()) {
-      m->sell_ws32 = 1;
-      m->sell_grid32 = sell_grid_for(m, 1, kSellBps);
-    }
+    if (m->sell_ws32 <= 2 && (long)nslices >= 24L * sm_count()) m->sell_ws32 = 1;
   } else if (sell_uses_deltas(m->sell_variant32)) {
     m->sell_variant32 = V_U8;
   }
+  default_sell_grids(m);
   DG_CUDA(cudaStreamSynchronize(st));
   m->sell_checkpoints = (long)nchk;
 }
@@ -593,13 +600,7 @@ SellShape choose_sell_shape(long n, int nslices, long stored, bool f32) {
   // fits one 16-element group, and the pipelined form, which has no second group to overlap, is the
   // slowest (12-14 % behind).
   const int var = per_row < 24.0 || (w >= 4 && per_row / w >= 32.0) ? V_U16 : V_PIPE8;
-  const int groups = kWarps / w;
-  const long need = (nslices + groups - 1) / groups;
-  // The pipelined form runs three blocks a SM (78 registers): one wave of blocks that walk the slices
-  // beats several (Hubbard m=512 126 against 130 us, Kondo m=127 16.9 against 17.4) and leaves a
-  // quarter of the reduction partials for the next kernel to sum.
-  const int bps = !f32 && var == V_PIPE8 ? kSellBpsPipe : kSellBps;
-  return SellShape{w, var, (int)std::max(1L, std::min(need, (long)sm_count() * bps))};
+  return SellShape{w, var};
 }
 
 dg_matrix *matrix_from_device(int n, long nnz_in, const long *row_d, const int *col_d, const double *val_d, int storage,
@@ -767,6 +768,7 @@ int dg_matrix_set_sell_shape(dg_matrix *m, int warps_per_slice, int grid) {
     m->sell_ws32 = warps_per_slice;
     m->sell_grid = grid;
     m->sell_grid32 = grid;
+    m->sell_grid_given = true;
     m->format = DG_FORMAT_SELL;
   });
 }
@@ -944,8 +946,8 @@ void profile_apply(dg_matrix *m, const XT *x_dev, double *y_dev, int iters, size
 // Matrices of one class (the same floor(log2 n), stored elements a row rounded, FP32 values or
 // not) share a launch shape.  The first matrix of a class is timed over every sliced-ELL
 // configuration: warps per slice x variant x grid for the FP64 product, then warps per slice x
-// variant of the FP32 product at that grid (the consumers of the products' reduction partials
-// count one per block, so both products keep one grid).  Only sliced-ELL shapes are candidates:
+// variant of the FP32 product, whose grid stays the default of its warps per slice.  Only sliced-ELL
+// shapes are candidates:
 // the lock-step batch runs on that layout.  The timings run next to whatever else the device is
 // doing (the engine's other jobs), so each candidate takes the better of two rounds and replaces
 // the build heuristic's shape only when at least 5 % faster.  The result is kept for the process.
@@ -957,7 +959,7 @@ struct ShapeClass {
 };
 struct TunedShape {
   int ws, variant, ws32, variant32;
-  int bps;   // the grid is min(blocks the slices need, bps blocks a SM)
+  int bps;   // the FP64 grid is min(blocks the slices need, bps blocks a SM)
 };
 std::mutex g_shape_mu;
 std::map<ShapeClass, TunedShape> g_shapes;
@@ -981,9 +983,10 @@ void apply_shape(dg_matrix *m, const TunedShape &t) {
   m->format = DG_FORMAT_SELL;
   m->sell_ws = t.ws;
   m->sell_variant = runnable_variant(m, t.variant);
-  m->sell_grid = m->sell_grid32 = sell_grid_for(m, t.ws, t.bps);
   m->sell_ws32 = t.ws32;
   m->sell_variant32 = runnable_variant(m, t.variant32);
+  default_sell_grids(m);
+  m->sell_grid = sell_grid_for(m, t.ws, t.bps);
 }
 
 TunedShape tune_sell(dg_matrix *m, int iters) {
@@ -1024,13 +1027,14 @@ TunedShape tune_sell(dg_matrix *m, int iters) {
   };
   // the build heuristic's shape first
   m->format = DG_FORMAT_SELL;
-  TunedShape best{m->sell_ws, m->sell_variant, m->sell_ws32, m->sell_variant32, m->sell_variant == V_PIPE8 ? kSellBpsPipe : kSellBps};
-  m->sell_grid = m->sell_grid32 = sell_grid_for(m, best.ws, best.bps);
+  TunedShape best{m->sell_ws, m->sell_variant, m->sell_ws32, m->sell_variant32, sell_bps(m->sell_variant)};
+  apply_shape(m, best);
   float best_ms = time_it(false);
   for (int ws = 1; ws <= 8; ws <<= 1)
     for (int v = 0; v < V_COUNT; ++v) {
       if (!candidate(ws, v)) continue;
-      for (int bps : {8, 16}) {
+      for (int bps : {kSellBpsPipe, 8, 16}) {
+        if (bps == kSellBpsPipe && v != V_PIPE8) continue;
         m->sell_ws = ws;
         m->sell_variant = v;
         m->sell_grid = sell_grid_for(m, ws, bps);
@@ -1051,6 +1055,7 @@ TunedShape tune_sell(dg_matrix *m, int iters) {
         if (!candidate(ws, v)) continue;
         m->sell_ws32 = ws;
         m->sell_variant32 = v;
+        m->sell_grid32 = sell_grid_for(m, ws, kSellBps);
         const float t = time_it(true);
         if (t < kGain * best_ms) {
           best_ms = t;
@@ -1087,6 +1092,7 @@ int dg_matrix_set_sell_window(dg_matrix *m, int window) {
     // a rebuilt layout without the delta stream falls back to 8-element groups
     m->sell_variant = (sell_uses_deltas(var) && !m->has_d16()) ? V_U8 : var;
     m->sell_variant32 = (sell_uses_deltas(var32) && !m->has_d16()) ? V_U8 : var32;
+    default_sell_grids(m);
     m->format = DG_FORMAT_SELL;
   });
 }
@@ -1110,6 +1116,7 @@ int dg_matrix_set_sell_variant(dg_matrix *m, int variant) {
                "variant %d needs the 16-bit column stream, which this matrix does not have", variant);
     m->sell_variant = variant;
     m->sell_variant32 = variant;
+    if (!m->sell_grid_given) default_sell_grids(m);
   });
 }
 
@@ -1123,6 +1130,7 @@ int dg_matrix_set_sell_mixed(dg_matrix *m, int warps_per_slice, int variant) {
                "variant %d needs the 16-bit column stream, which this matrix does not have", variant);
     m->sell_ws32 = warps_per_slice;
     m->sell_variant32 = variant;
+    if (!m->sell_grid_given) m->sell_grid32 = sell_grid_for(m, warps_per_slice, kSellBps);
   });
 }
 
@@ -1222,6 +1230,7 @@ int dg_matrix_autotune(dg_matrix *m, int iters, dg_tune_result *out) {
       m->sell_ws32 = best.shape;
       m->sell_variant = best.variant;
       m->sell_grid = m->sell_grid32 = best.grid;
+      m->sell_grid_given = true;
       if (sell_uses_deltas(m->sell_variant32) && !m->has_d16()) m->sell_variant32 = V_U8;
     } else {
       m->format = DG_FORMAT_CSR;

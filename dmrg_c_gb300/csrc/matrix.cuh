@@ -24,6 +24,7 @@ struct dg_matrix {
   long nnz_sell = 0;               // stored elements including padding
   int sell_grid = 1;
   int sell_grid32 = 1;             // grid of the FP32 (mixed) product
+  bool sell_grid_given = false;    // the grids are the caller's or the autotuner's, not the defaults of the shapes
   int sell_ws = 1;                 // warps per slice
   int sell_ws32 = 1;               // warps per slice of the FP32 (mixed) product
   int sell_variant = 1;            // SellVariant of the FP64 product (V_U8)
@@ -133,10 +134,10 @@ void launch_sell(const SellOp<VT> &op, int grid, const XT *x, Scale sc, double s
   DG_CUDA(cudaGetLastError());
 }
 
-// Warps per slice, variant and grid of the sliced-ELL kernel for n rows with `stored` elements
+// Warps per slice and variant of the sliced-ELL kernel for n rows with `stored` elements
 // (matrix.cu; heuristic from measured sweeps).
 struct SellShape {
-  int ws, variant, grid;
+  int ws, variant;
 };
 SellShape choose_sell_shape(long n, int nslices, long stored, bool f32);
 

@@ -199,10 +199,11 @@ int dg_matrix_set_sell_shape(dg_matrix *m, int warps_per_slice, int grid);
  * delta stream (with more warps per slice it runs variant 5).  Variants 5 and 6 need the delta
  * stream (dg_matrix_sell_deltas; DG_ERR_ARG otherwise).  The FP64 product's default is 3, or
  * 2 for short rows (< 24 stored a row) and for 4-8 warps a slice of >= 32 elements each; the FP32
- * (mixed) product's is 1, or 5 with the delta stream; this call sets both. */
+ * (mixed) product's is 1, or 5 with the delta stream; this call sets both.  The grids become the
+ * defaults for the new variant, unless dg_matrix_set_sell_shape or dg_matrix_autotune set them. */
 int dg_matrix_set_sell_variant(dg_matrix *m, int variant);
-/* Warps per slice and variant of the FP32 (mixed-precision) product alone; its grid stays (the
- * default's, or that of dg_matrix_set_sell_shape, which sets both products). */
+/* Warps per slice and variant of the FP32 (mixed-precision) product alone; its grid becomes the
+ * default for them, unless dg_matrix_set_sell_shape or dg_matrix_autotune set it. */
 int dg_matrix_set_sell_mixed(dg_matrix *m, int warps_per_slice, int variant);
 /* *present = 1 if the sliced-ELL copy carries the 16-bit column-delta stream (built for
  * matrices with FP32 values (DG_VALUES_F32 / DG_VALUES_BOTH) of at least 4M stored elements
@@ -240,8 +241,8 @@ int dg_matrix_autotune(dg_matrix *m, int iters, dg_tune_result *out);
  * autotuner).  A class is floor(log2 n), the stored elements a row rounded, and whether the
  * matrix has FP32 values.  If m's class has a tuned shape it is applied to m (*how = 1).  Else,
  * with tune != 0 and no other thread tuning the class, m is timed over every sliced-ELL
- * configuration (warps per slice x variant x grid of 8 or 16 blocks a SM for the FP64 product,
- * then warps per slice x variant of the FP32 product at that grid; iters launches each), the
+ * configuration (warps per slice x variant x grid of 8 or 16 blocks a SM, variant 3 also of 3, for
+ * the FP64 product, then warps per slice x variant of the FP32 product; iters launches each), the
  * fastest is applied and recorded for the class (*how = 2).  Otherwise m keeps its shape
  * (*how = 0).  The timings run on the calling thread's stream and see whatever else the device
  * is doing. */
