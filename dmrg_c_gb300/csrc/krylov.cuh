@@ -239,16 +239,42 @@ struct EpiLzRaw {
   __device__ void finalize(double) const {}
 };
 
-// Step b on w_b (unnormalised; w_0 normalised) and y = H w_b: beta_b = ||w_b|| (b > 0: from the previous
-// step's vcount partials in rp; O[b] = beta_b, 0 for b = 0), v_b = w_b / beta_b into v, alpha_b =
-// <y, w_b> / beta_b^2 (the product's pcount partials in pp; D[b]), then
-// w_{b+1} = y / beta_b - alpha_b v_b - beta_b v_{b-1} (sml/LANCZOS_SYM.c:121-143, 240-243) into w, block
-// partials of <w,w> into wp.  Block 0 records D, O and their host mirrors.
+// The power of two just below sqrt(x), kept where its inverse is a normal number too; 1 for an x that is
+// not positive and finite.
+__device__ __forceinline__ double pow2_root(double x) {
+  const long long e = (__double_as_longlong(x) >> 52) & 0x7ff;
+  return x > 0.0 && e < 0x7ff ? __longlong_as_double((1023 + ((e - 1023) >> 1)) << 52) : 1.0;
+}
+// 1/g of a power of two from pow2_root
+__device__ __forceinline__ double pow2_inverse(double g) { return __longlong_as_double((2046ll << 52) - __double_as_longlong(g)); }
+
+// Block partials of <x,x>.
+template <int T>
+__global__ void __launch_bounds__(T) k_sq_partials(int n, const double *__restrict__ x, double *part) {
+  pdl_wait();
+  double t[1] = {0.0};
+  for (int i = blockIdx.x * T + threadIdx.x; i < n; i += gridDim.x * T) t[0] += x[i] * x[i];
+  pdl_trigger();
+  block_sums<T, 1>(t);
+  if (threadIdx.x == 0) part[blockIdx.x] = t[0];
+}
+
+// Step b on w_b and y = H w_b.  w_0 is normalised; from step 1 on w_b is the unnormalised Krylov
+// vector over a power of two G of the cycle, that of ||H w_0||: with the vector itself, of norm up to
+// ||H||, the sum <y, w_b> is of the order of ||H||^3 and leaves the double range at ||H|| = 1e102 (over
+// G at about 1e150, where <w,w> did in any form); a power of two changes no bit of the other numbers.
+// Cost: the sum <y,y> of step 0 and one more factor, 0.3 - 1 % of the XXZ m=64 solve.
+//   beta_b = G ||w_b|| (b > 0: from the previous step's rcount partials in rp; O[b] = beta_b, 0 for b = 0),
+//   v_b = w_b / ||w_b|| into v, alpha_b = <y, w_b> / ||w_b||^2 (the product's pcount partials in pp; D[b]),
+//   w_{b+1} = (y / ||w_b|| - alpha_b v_b - beta_b v_{b-1}) / G
+//   (sml/LANCZOS_SYM.c:121-143, 240-243) into w, block partials of <w,w> into wp.
+// scale: *scale = G, which step 0 forms from <y,y> (its partials in rp).  Block 0 records D, O, G and the host mirrors.
 template <int T>
 __global__ void __launch_bounds__(T) k_lz_step(int n, const double *__restrict__ y, double *__restrict__ w, double *__restrict__ v,
-                                              const double *__restrict__ vprev, double *D, double *O, double *hD, double *hO, int b,
-                                              const double *pp, int pcount, const double *rp, int rcount, double *wp) {
-  __shared__ double s_sc[3];
+                                              const double *__restrict__ vprev, double *D, double *O, double *scale, double *hD,
+                                              double *hO, int b, const double *pp, int pcount, const double *rp, int rcount,
+                                              double *wp) {
+  __shared__ double s_sc[4];
   pdl_wait();
   // the first elements' operands are loaded before the partial sums, so that the L2 round trips overlap
   const int i0 = blockIdx.x * T + threadIdx.x, stride = gridDim.x * T;
@@ -262,31 +288,35 @@ __global__ void __launch_bounds__(T) k_lz_step(int n, const double *__restrict__
     w0[u] = in ? w[i] : 0.0;
     p0[u] = in && b > 0 ? vprev[i] : 0.0;
   }
+  const double s0 = b > 0 ? __ldcg(scale) : 0.0;
   {
-    double t[2] = {partials_share(pp, pcount), b > 0 ? partials_share(rp, rcount) : 0.0};
+    double t[2] = {partials_share(pp, pcount), partials_share(rp, rcount)};
     block_sums<T, 2>(t);
     if (threadIdx.x == 0) {
-      const double o = b > 0 ? sqrt(t[1]) : 0.0, sc = b > 0 ? 1.0 / o : 1.0;
-      const double d = t[0] * sc * sc;
+      const double g = b > 0 ? s0 : pow2_root(t[1]), f = pow2_inverse(g);
+      const double nw = b > 0 ? sqrt(t[1]) : 0.0, sc = b > 0 ? 1.0 / nw : 1.0;
+      const double scf = sc * f, d = t[0] * sc * scf;
       s_sc[0] = d;
-      s_sc[1] = o;
+      s_sc[1] = nw;
       s_sc[2] = sc;
+      s_sc[3] = scf;
       if (blockIdx.x == 0) {
-        D[b] = d;
-        O[b] = o;
-        hD[b] = d;
-        hO[b] = o;
+        const double alpha = d * g, beta = nw * g;
+        D[b] = alpha;
+        O[b] = beta;
+        if (b == 0) *scale = g;
+        hD[b] = alpha;
+        hO[b] = beta;
       }
     }
   }
   __syncthreads();
-  const double d = s_sc[0], o = s_sc[1], sc = s_sc[2];
+  const double d = s_sc[0], o = s_sc[1], sc = s_sc[2], scf = s_sc[3];   // alpha / G, beta / G, of w, of y
   double acc = 0.0;
   auto step = [&](int i, double yi, double wi, double pi) {
-    const double vi = b > 0 ? wi * sc : wi;
-    if (b > 0) yi *= sc;
-    double r = yi - d * vi;
-    if (b > 0) r = r - o * pi;
+    const double vi = wi * sc;
+    double r = __fma_rn(-d, vi, __dmul_rn(yi, scf));
+    if (b > 0) r = __fma_rn(-o, pi, r);
     v[i] = vi;
     w[i] = r;
     acc += r * r;
@@ -702,10 +732,10 @@ struct LzSteps64 {
   Workspace &ws;
   LzState &z;
   double *w;             // start vector in, next unnormalised Krylov vector
-  DevBuf<double> y, c;
+  DevBuf<double> y, c, g;   // g: the power of two that a cycle's Krylov vectors are divided by
   KrylovBasis<double> B;
   LzSteps64(const Opl &o, const LanczosCfg &cf, Workspace &w_, LzState &z_, double *w_dev)
-      : op(o), cfg(cf), ws(w_), z(z_), w(w_dev), y(z_.n), c(z_.cap_max + 1), B(z_.n, w_.st) {}
+      : op(o), cfg(cf), ws(w_), z(z_), w(w_dev), y(z_.n), c(z_.cap_max + 1), g(1), B(z_.n, w_.st) {}
   void begin_cycle() {
     if (cfg.reorth) return;
     k_scale_rsqrt<double><<<ws.vgrid, kThreads, 0, ws.st>>>(w, z.n, &ws.S()->r2); ::dg::count_launch();
@@ -723,8 +753,11 @@ struct LzSteps64 {
       op.apply(w, Scale{}, 0.0, (const int *)nullptr, EpiLzRaw{y.get()}, slot, st);
       // <w,w> partials alternate: a step reads the last one's while it writes its own
       double *const rp[2] = {ws.partials2.get(), ws.partials3.get()};
+      if (b == 0)   // <y,y>, the scale of the cycle
+        launch_pdl(ws.uthreads == kThreads ? k_sq_partials<kThreads> : k_sq_partials<512>, ws.ugrid, ws.uthreads, st, n,
+                   (const double *)y.get(), rp[1]);
       launch_pdl(ws.uthreads == kThreads ? k_lz_step<kThreads> : k_lz_step<512>, ws.ugrid, ws.uthreads, st, n, (const double *)y.get(),
-                 w, B.vec(b), vprev, z.D.get(), z.O.get(), z.hD.d, z.hO.d, b, (const double *)slot.partials, op.grid(),
+                 w, B.vec(b), vprev, z.D.get(), z.O.get(), g.get(), z.hD.d, z.hO.d, b, (const double *)slot.partials, op.grid(),
                  (const double *)rp[(b + 1) & 1], ws.ugrid, rp[b & 1]);
       return;
     }
