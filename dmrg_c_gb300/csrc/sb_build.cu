@@ -467,11 +467,13 @@ dg_sb *sb_build(const dg_sb_model *m, const SbBasisView *bv) {
     DG_CUDA(cudaStreamSynchronize(st));
     int cap = 32;
     while (cap < hmost) cap <<= 1;
-    // warps a block bounded by 192 KB of shared memory (cap <= 4096: three warps at least)
+    // warps a block bounded by 192 KB of shared memory (cap <= 4096: three warps at least); the limit is
+    // set to that for every superblock, since all threads that build one share it
+    constexpr size_t kMost = 192 << 10;
     const size_t per_warp = (size_t)cap * (sizeof(uint64_t) + sizeof(double));
-    const int warps = (int)std::min<size_t>(kSbWarps, (192u << 10) / per_warp);
+    const int warps = (int)std::min<size_t>(kSbWarps, kMost / per_warp);
     const size_t smem = per_warp * warps;
-    DG_CUDA(cudaFuncSetAttribute(k_sb_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    DG_CUDA(cudaFuncSetAttribute(k_sb_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
     const long blocks = std::max(1L, std::min<long>((n + warps - 1) / warps, (long)sm_count() * 32));
     DevBuf<int> scol;
     DevBuf<double> sval;
