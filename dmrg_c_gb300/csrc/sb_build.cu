@@ -501,8 +501,24 @@ dg_sb *sb_build(const dg_sb_model *m, const SbBasisView *bv) {
     DG_CUDA(cudaStreamSynchronize(st));
     DG_REQUIRE(herr == 0, DG_ERR_INTERNAL, "superblock row generation overflowed its buffer");
     s->nnz = total;
-    s->col.alloc(total);
-    s->val.alloc(total);
+    auto take_result = [&] {
+      s->col.alloc(total);
+      s->val.alloc(total);
+    };
+    try {
+      take_result();
+    } catch (const Error &e) {
+      if (e.code != DG_ERR_NOMEM || !single) throw;
+      // no room for the result beside the scratch: it takes the scratch's place (a row keeps no more than it
+      // generates) and the fill pass generates the rows again
+      cudaGetLastError();
+      s->col.release();
+      scol.release();
+      sval.release();
+      soff.release();
+      single = false;
+      take_result();
+    }
     if (single) {
       k_sb_compact<<<(int)std::max(1L, std::min<long>((n + kWarps - 1) / kWarps, (long)sm_count() * 16)), kThreads, 0, st>>>(
           n, soff.get(), s->row.get(), scol.get(), sval.get(), s->col.get(), s->val.get()); ::dg::count_launch();
