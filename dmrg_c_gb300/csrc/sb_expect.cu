@@ -587,12 +587,14 @@ bool trace_form(const dg_sb_basis *b, const std::vector<SbTerm> &terms, long v_l
   return true;
 }
 
-void launch_trace(const dg_sb_basis *b, const std::vector<SbTerm> &terms, const dg_sb_ops *ops, const double *v, const double *w0,
-                  const double *w1, double *dout, cudaStream_t st) {
+// Enqueues the density-matrix form of the terms.  tt: their host list for the device, the caller's, kept until
+// the stream has drained (it is uploaded from there).
+void launch_trace(const dg_sb_basis *b, const std::vector<SbTerm> &terms, std::vector<TraceTerm> &tt, const dg_sb_ops *ops,
+                  const double *v, const double *w0, const double *w1, double *dout, cudaStream_t st) {
   const SbPairs &P = *b->pairs;
   const PairView pv = pair_view(P);
   int need[2] = {0, 0};   // of each weight vector's density matrices
-  std::vector<TraceTerm> tt;
+  tt.clear();
   for (const SbTerm &t : terms) {
     need[t.weight] |= t.pos == DG_SB_LL ? kNeedLL : t.pos == DG_SB_LR ? kNeedLR : t.pos == DG_SB_RR ? kNeedRR : kNeedRL;
     tt.push_back(TraceTerm{t.row, t.pos, t.weight});
@@ -637,7 +639,8 @@ void launch_expect(const SbStates &S, const int *inv, const SbGeom &g, const std
   DG_REQUIRE(nt <= 65535, DG_ERR_ARG, "at most 65535 terms per call (got %d)", nt);
   if (trace_form(one_sector, terms, v_len)) {
     DevBuf<double> dout(nt);
-    launch_trace(one_sector, terms, ops, v, w0, w1, dout.get(), st);
+    std::vector<TraceTerm> tt;
+    launch_trace(one_sector, terms, tt, ops, v, w0, w1, dout.get(), st);
     DG_CUDA(cudaMemcpyAsync(out_host, dout.get(), sizeof(double) * nt, cudaMemcpyDeviceToHost, st));
     DG_CUDA(cudaStreamSynchronize(st));
     return;
