@@ -39,39 +39,31 @@ __device__ __forceinline__ void set_norm2(Norm2 *p, double t) {
 // root or division is a long sequence of FP64 instructions; on GB300's few FP64 pipes,
 // evaluated by every thread of a product it costs as much FP64 issue as the product's
 // multiply-adds, so it is formed once: by the last block of the kernel that reduced <w,w>
-// (NORM2), or, when that kernel left block partials, once per block of the product (PARTIALS).
+// (NORM2), or, when that kernel left block partials (FP32 pairs: the mixed form), once per block of the
+// product (PAIRS).
 //   ONE       s = 1
 //   MUL       s = *p                       (MINIMUM_RESIDUAL: 1/gamma0)
 //   NORM2     s = rs of the Norm2 at p      (NORMALIZE: 1/sqrt(<w,w>)), r2 = its v
-//   PARTIALS  r2 = sum of count block partials at p, s = 1/sqrt(r2)
+//   PAIRS     r2 = sum of count block partials at p (float2, sum_partials_pair), s = 1/sqrt(r2)
 struct Scale {
-  // PAIRS: as PARTIALS, the partials being FP32 pairs (float2, sum_partials_pair; the mixed form)
-  enum Mode : int { ONE = 0, MUL = 1, NORM2 = 2, PARTIALS = 3, PAIRS = 4 };
+  enum Mode : int { ONE = 0, MUL = 1, NORM2 = 2, PAIRS = 3 };
   const double *p = nullptr;
   int mode = ONE;
   int count = 0;
   static Scale mul(const double *q) { return Scale{q, MUL, 0}; }
   static Scale norm2(const Norm2 *q) { return Scale{reinterpret_cast<const double *>(q), NORM2, 0}; }
-  static Scale partials(const double *q, int c) { return Scale{q, PARTIALS, c}; }
   static Scale pairs(const double *q, int c) { return Scale{q, PAIRS, c}; }
 };
 
 struct ScaleVal {
   double s;
-  double r2;   // <w,w> behind s (NORM2, PARTIALS), else 0
+  double r2;   // <w,w> behind s (NORM2, PAIRS), else 0
 };
 
-// Every thread of the block must call it (PARTIALS synchronises the block).
+// Every thread of the block must call it (PAIRS synchronises the block).
 __device__ __forceinline__ ScaleVal load_scale(const Scale &sc) {
   if (sc.mode == Scale::MUL) return ScaleVal{*sc.p, 0.0};
   if (sc.mode == Scale::NORM2) return ScaleVal{sc.p[1], sc.p[0]};
-  if (sc.mode == Scale::PARTIALS) {
-    __shared__ double s_rs;
-    const double r2 = sum_partials(sc.p, sc.count);
-    if (threadIdx.x == 0) s_rs = 1.0 / sqrt(r2);
-    __syncthreads();
-    return ScaleVal{s_rs, r2};
-  }
   if (sc.mode == Scale::PAIRS) {
     // FP32 merges in every thread; the FP64 square root and division once, in thread 0
     __shared__ double s_rs2, s_r22;

@@ -628,7 +628,6 @@ __global__ void k_mr_update(int n, const double *__restrict__ v1n, const double 
 //   int grid() const;   // apply grid (workspace sizing; number of block partials a product leaves)
 //   int grid32() const; // the same of the FP32 product
 //   const dg_matrix *matrix() const;   // the CRS behind the operator, null if there is none
-//   long nnz() const;   // stored elements (or an estimate; 0 if unknown)
 // ---------------------------------------------------------------------------------
 
 struct LanczosResult {
@@ -813,7 +812,7 @@ struct LzStepsMixed {
     Scalars *S = ws.S();
     const RedSlot slot = ws.slot();
     B.ensure(b + 2, z.cap_max);
-    // as LzSteps64: reductions finished by the consumer on products with enough work a block
+    // the reductions' partials are left to their consumers (lz_defer_mixed)
     const bool defer = lz_defer_mixed();
     const Scale sc = (b > 0 && defer) ? Scale::pairs(ws.partials2.get(), ws.vgrid) : Scale::norm2(&S->r2);
     if (defer) {

@@ -80,7 +80,6 @@ struct RawCrsLauncher {
   int grid() const { return grid_; }
   int grid32() const { return grid_; }
   const dg_matrix *matrix() const { return nullptr; }
-  long nnz() const { return 0; }
   template <class XT, class Epi>
   void apply(const XT *x, Scale sc, double sigma, const int *gate, const Epi &epi, RedSlot slot,
              cudaStream_t st) const {

@@ -124,7 +124,6 @@ struct ObcLauncher {
   int grid() const { return D->grid; }
   int grid32() const { return D->grid; }
   const dg_matrix *matrix() const { return nullptr; }
-  long nnz() const { return (long)D->n * D->nnz_est; }   // nnz_est: elements a row
   template <class XT, class Epi>
   void apply(const XT *x, Scale sc, double sigma, const int *gate, const Epi &epi, RedSlot slot,
              cudaStream_t st) const {

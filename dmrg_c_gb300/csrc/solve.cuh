@@ -28,7 +28,6 @@ struct CrsLauncher {
   int grid() const { return matrix_grid(m); }
   int grid32() const { return matrix_grid32(m); }
   const dg_matrix *matrix() const { return m; }
-  long nnz() const { return m->nnz; }
   template <class XT, class Epi>
   void apply(const XT *x, Scale sc, double sigma, const int *gate, const Epi &epi, RedSlot slot,
              cudaStream_t st) const {
