@@ -282,6 +282,29 @@ void mapped_return(void *h, size_t bytes) {
   cudaFreeHost(h);   // (waits for the device)
 }
 
+// What the lists hold idle goes back: the pinned blocks and the current device's streams.
+static void release_idle() {
+  std::vector<MappedBlock> blocks;
+  {
+    MappedList &l = mapped_list();
+    std::lock_guard<std::mutex> lk(l.mu);
+    l.collect();
+    blocks.swap(l.idle);
+    for (const MappedBlock &b : blocks) l.bytes -= b.bytes;
+  }
+  for (const MappedBlock &b : blocks) cudaFreeHost(b.h);
+  int dev = 0;
+  DG_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= kMaxPoolDevices) return;
+  std::vector<cudaStream_t> streams;
+  {
+    IdleStreams &is = idle_streams();
+    std::lock_guard<std::mutex> lk(is.mu);
+    streams.swap(is.idle[dev]);
+  }
+  for (cudaStream_t s : streams) cudaStreamDestroy(s);   // (work still queued on one runs to its end)
+}
+
 int sm_count() {
   thread_local int cached = -1, dev = -1;
   int cur = 0;
@@ -385,6 +408,7 @@ int dg_release_pool(void) {
     dg::require_device();
     DG_CUDA(cudaStreamSynchronize(dg::stream()));
     DG_CUDA(cudaMemPoolTrimTo(dg::device_pool(), 0));
+    dg::release_idle();
   });
 }
 

@@ -162,8 +162,10 @@ long dg_kernel_launches(void);
 
 /* Device memory the library allocates comes from its own stream-ordered pool, one per
  * device; freed blocks stay cached (up to DG_POOL_KEEP_MB, default 8192) so repeated solves
- * do not call cudaMalloc / cudaFree.  dg_release_pool returns the cached blocks of the
- * current device to the system.  (No counterpart in the reference.) */
+ * do not call cudaMalloc / cudaFree.  Pinned host blocks (at most 64 MiB) and the streams of threads
+ * that ended (at most 64 a device) are kept for later calls too.  dg_release_pool returns the cached
+ * blocks and streams of the current device, and the pinned blocks, to the system.  (No
+ * counterpart in the reference.) */
 int dg_release_pool(void);
 
 /* Opaque device-resident sparse operator (full CRS on the device, FP64 values and,
