@@ -22,7 +22,8 @@ constexpr int kCgThreads = 512;
 // Sizes up to which the cluster is faster than the three kernels on the whole GPU, whose 11 - 12 us an
 // iteration do not depend on the size there.  Measured, us an iteration on the cluster (n, elements):
 // 5.8 (100, 1 k), 6.5 (924, 8 k), 9.0 (3,432, 31 k), 10.1 (2,000, 62 k); past the limits 13.9 (8,000, 72 k) and
-// 16.2 (3,696, 245 k), bound by the FP64 issue of 16 SMs.
+// 16.2 (3,696, 245 k; 4.4 of it FP64 issue of 16 SMs, the rest their gathers and barriers).  At 3,432 rows the
+// FP64 pipe is 31 % busy and most stalls are at barriers.
 constexpr int kCgClusterN = 4096;
 constexpr long kCgClusterNnz = 1L << 16;
 

@@ -6,7 +6,8 @@
 // owns a contiguous range of rows, holds its part of the basis in shared memory (read once for the
 // four passes over it, and before the kernel waits for its predecessor, except for the newest
 // vector), and the reductions are exchanged through distributed shared memory, one cluster barrier
-// each: alpha, the coefficients of each pass, the norm.  FP64 issue bounds what is left (19 cycles a
+// each: alpha, the coefficients of each pass, the norm.  What is left is latency: barriers, the
+// chains of dependent FP64 operations and loads (the FP64 pipe of a CTA's SM is 31 % busy, at 19 cycles a
 // warp instruction): the dot products are summed by transposing through shared memory (one add a
 // lane and vector instead of a five-step shuffle tree), the subtraction by four threads a row.
 //
