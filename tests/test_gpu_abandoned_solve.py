@@ -1,6 +1,6 @@
 """A solve that gives up while its kernels are still queued, beside solves on other threads: what it
 leaves behind (its pinned blocks, and with its thread its stream) must not reach them before its last
-kernel has run.  Runs in a process of its own with a short bound on the waits (5 ms); the solve that gives
+kernel has run.  Runs in a process of its own with a short bound on the waits (20 ms); the solve that gives
 up has a product of one block (62 ms), and the others wait some tens of microseconds.  All kernels are
 loaded beforehand (loading one waits for the kernels that run) and every stream has a work queue of its
 own."""
@@ -71,7 +71,7 @@ print("ok")
 
 @pytest.mark.parametrize("thread", ["stays", "ends"])
 def test_abandoned_solve(gpu, thread):
-    env = dict(os.environ, DG_WAIT_TIMEOUT_MS="5", CUDA_MODULE_LOADING="EAGER", CUDA_DEVICE_MAX_CONNECTIONS="32",
+    env = dict(os.environ, DG_WAIT_TIMEOUT_MS="20", CUDA_MODULE_LOADING="EAGER", CUDA_DEVICE_MAX_CONNECTIONS="32",
                PYTHONPATH=str(ROOT))
     r = subprocess.run([sys.executable, "-c", SCRIPT, thread], cwd=ROOT, env=env, capture_output=True, text=True, timeout=120)
     print(r.stdout)
